@@ -320,7 +320,8 @@ typedef struct {
     int mode;
     int rows_static;            /* row capacity of A and D; the row count when num_rows is NULL */
     int row_begin, row_end;     /* modes 0-2: only rows [row_begin, min(row_end, rows)) are computed; row_end = 0 means all.
-                                   Both must be multiples of 256. */
+                                   Both must be multiples of 256.  Mode 3: A and B hold rows [row_begin,
+                                   row_begin + rows_static) of group_offsets' numbering (row_end unused) */
     const int32_t* num_rows;    /* device, optional */
     const int32_t* group_of_block;   /* device [rows/128], optional */
     const int32_t* group_offsets;    /* device [G+1] (mode 3) */

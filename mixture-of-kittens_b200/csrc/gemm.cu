@@ -68,7 +68,7 @@ struct Geo {
 
 struct KParams {
     int rows_cap;                    // static upper bound of rows
-    int row_begin, row_end;          // row window (multiples of 256); row_end <= rows_cap
+    int row_begin, row_end;          // row window (multiples of 256); row_end <= rows_cap.  MODE_WGRAD: row_begin = number of the operands' first row
     const int32_t* num_rows;         // device, optional
     const int32_t* group_of_block;   // device [rows/128], optional
     const int32_t* group_offsets;    // device [G+1], MODE_WGRAD
@@ -360,7 +360,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll
                         for (int c = 0; c < G::B_COLS / 64; ++c) tma_tile<NCTA>(b_dst + c * CHUNK_BYTES, tb, fb, bcol0 + 64 * c, brow);
                     } else {
-                        const int krow = ti.k_row0 + it * BK;
+                        const int krow = ti.k_row0 - p.row_begin + it * BK;
 #pragma unroll
                         for (int c = 0; c < 2; ++c) tma_tile<NCTA>(a_dst + c * CHUNK_BYTES, &tmA, fb, row0 + 64 * c, krow);
 #pragma unroll
@@ -683,7 +683,8 @@ extern "C" int mokb_grouped_gemm_bf16(const mokb_gemm_args* g, void* stream_) {
     p.rows_cap = g->rows_static;
     p.row_begin = g->row_begin;
     p.row_end = g->row_end > 0 ? g->row_end : g->rows_static;
-    MOKB_REQUIRE(p.row_begin >= 0 && p.row_begin % 256 == 0 && p.row_end % (128 * ncta) == 0 && p.row_begin <= p.row_end && p.row_end <= g->rows_static,
+    MOKB_REQUIRE(p.row_begin >= 0 && p.row_begin % 256 == 0, "grouped_gemm: row_begin must be a non-negative multiple of 256");
+    MOKB_REQUIRE(g->mode == MODE_WGRAD || (p.row_end % (128 * ncta) == 0 && p.row_begin <= p.row_end && p.row_end <= g->rows_static),
                  "grouped_gemm: bad row window [%d, %d) of %d", g->row_begin, g->row_end, g->rows_static);
     p.num_rows = g->num_rows;
     p.group_of_block = g->group_of_block;
@@ -797,6 +798,10 @@ extern "C" int mokb_grouped_gemm_bf16(const mokb_gemm_args* g, void* stream_) {
     default: {
         MOKB_REQUIRE(g->M > 0 && g->M % 128 == 0 && g->N > 0 && g->N % 64 == 0, "grouped_gemm WGRAD: M %% 128 and N %% 64 must be 0");
         MOKB_REQUIRE(g->group_offsets != nullptr, "grouped_gemm WGRAD: group_offsets required");
+        // The maps start at the buffers themselves and the coordinates count from row_begin.  (A map moved back by row_begin
+        // rows, as the row-tiled modes use, would have a base outside the buffer: harmless for boxes inside the tensor, but
+        // here the boxes of a partial last tile (M or N not a multiple of 256) lie entirely outside of it, and such a box
+        // on a base that is not mapped memory is an illegal memory access.)
         MOKB_TRY(make_tmap_2d(&ta, g->A, 2, g->M, rows, 2ull * g->lda, 64, 64));
         MOKB_TRY(make_tmap_2d(&tb, g->B, 2, g->N, rows, 2ull * g->ldb, 64, 64));
         ta2 = ta; tb2 = tb;

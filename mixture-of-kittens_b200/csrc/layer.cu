@@ -198,10 +198,11 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
     MOKB_TRY(run_prologue(a->tokens_per_expert, a->num_tokens, a->peer_rank, E_l, C, MB, T, s, a->status, stream));
     const void* d_y_local = reinterpret_cast<const void*>(static_cast<uintptr_t>(a->d_y_ptrs_host[a->ep_rank]));
     const void* x_local = reinterpret_cast<const void*>(static_cast<uintptr_t>(a->x_ptrs_host[a->ep_rank]));
-    auto wgrad = [&](const void* A, int M, const void* B, int N, void* D, int G, int rows, const int32_t* offs, int accumulate,
+    // A and B as they lie in memory: `rows` rows, the first of which is row `first` in the numbering of `offs`
+    auto wgrad = [&](const void* A, int M, const void* B, int N, void* D, int G, int first, int rows, const int32_t* offs, int accumulate,
                      const int32_t* k_end = nullptr) -> int {
         mokb_gemm_args w = gemm_base(a->status);
-        w.mode = 3; w.rows_static = rows; w.G = G; w.M = M; w.N = N; w.group_offsets = offs; w.accumulate = accumulate;
+        w.mode = 3; w.row_begin = first; w.rows_static = rows; w.G = G; w.M = M; w.N = N; w.group_offsets = offs; w.accumulate = accumulate;
         w.group_k_end = k_end;       // the padding rows at the end of every expert's segment are zero: not multiplied
         w.A = A; w.lda = M; w.B = B; w.ldb = N; w.D = D; w.ldd = N;
         return mokb_grouped_gemm_bf16(&w, stream);
@@ -257,9 +258,9 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
             g.A = a->d_gate_shared; g.B = a->w_shared_gate; g.A2 = a->d_up_shared; g.B2 = a->w_shared_up; g.lda = I; g.ldb = H;
             g.D = a->d_x_shared; g.ldd = H;
             MOKB_TRY(mokb_grouped_gemm_bf16(&g, stream));
-            MOKB_TRY(wgrad(d_y_local, H, a->hidden_shared, I, a->d_w_shared_down, 1, T, s.shared_offsets, 0));
-            MOKB_TRY(wgrad(a->d_gate_shared, I, x_local, H, a->d_w_shared_gate, 1, T, s.shared_offsets, 0));
-            MOKB_TRY(wgrad(a->d_up_shared, I, x_local, H, a->d_w_shared_up, 1, T, s.shared_offsets, 0));
+            MOKB_TRY(wgrad(d_y_local, H, a->hidden_shared, I, a->d_w_shared_down, 1, 0, T, s.shared_offsets, 0));
+            MOKB_TRY(wgrad(a->d_gate_shared, I, x_local, H, a->d_w_shared_gate, 1, 0, T, s.shared_offsets, 0));
+            MOKB_TRY(wgrad(a->d_up_shared, I, x_local, H, a->d_w_shared_up, 1, 0, T, s.shared_offsets, 0));
         }
 
         // ---- routed experts of this macrobatch
@@ -299,9 +300,9 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
         MOKB_TRY(mokb_grouped_gemm_bf16(&g, stream));
         const int32_t* offs = s.mb_offsets + static_cast<size_t>(m) * (E_l + 1);
         const int32_t* k_end = s.mb_k_end + static_cast<size_t>(m) * (E_l + 1);
-        MOKB_TRY(wgrad(d_y_r, H, hidden_r, I, a->d_w_routed_down, E_l, hi, offs, m > 0, k_end));
-        MOKB_TRY(wgrad(d_gate_r, I, x_routed, H, a->d_w_routed_gate, E_l, hi, offs, m > 0, k_end));
-        MOKB_TRY(wgrad(d_up_r, I, x_routed, H, a->d_w_routed_up, E_l, hi, offs, m > 0, k_end));
+        MOKB_TRY(wgrad(a->d_y_routed, H, a->hidden_routed, I, a->d_w_routed_down, E_l, lo, hi - lo, offs, m > 0, k_end));
+        MOKB_TRY(wgrad(a->d_gate_routed, I, a->x_routed, H, a->d_w_routed_gate, E_l, lo, hi - lo, offs, m > 0, k_end));
+        MOKB_TRY(wgrad(a->d_up_routed, I, a->x_routed, H, a->d_w_routed_up, E_l, lo, hi - lo, offs, m > 0, k_end));
     }
     return MOKB_OK;
 }
