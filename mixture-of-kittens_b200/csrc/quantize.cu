@@ -5,9 +5,10 @@
 //   (SwiGLU forward + quantise is the epilogue of the MXFP8 gate/up GEMM, gemm_mxfp8.cu)
 //   swiglu_bwd_quant_kernel de-quantise saved gate/up, SwiGLU backward, router-gradient partials,
 //                           quantise d_gate / d_up      (reference: swiglu.cuh:209-566)
-// One 128 x 128 tile per CTA, staged in shared memory as packed bf16 pairs with an odd word pitch,
-// so that the row-wise pass (a thread owns 32 columns of one row) and the column-wise pass (a
-// thread owns 32 rows of two adjacent columns) both read it without bank conflicts.  The kernels
+// One 128 x 128 tile per CTA.  A thread quantises 16 columns of a row straight from the registers it
+// loaded them into (the block maximum is shared with the neighbouring lane) and stages them in shared
+// memory as packed bf16 pairs; the column-wise pass (a thread owns 32 rows of two adjacent columns)
+// reads them back.  Both are free of bank conflicts, and every global access covers whole lines.  The kernels
 // are bound by HBM, but only if the per-element instruction count stays small: everything works on
 // bf16 pairs (packed abs/max for the block maximum, one conversion instruction per two outputs)
 // and global memory is touched 32 bytes per thread per instruction.
@@ -20,79 +21,65 @@ namespace mokb {
 namespace {
 
 constexpr int TILE = 128;
-constexpr int WPITCH = TILE / 2 + 1;          // 32-bit words per smem row (65: odd)
-constexpr int TILE_WORDS = TILE * WPITCH;
+constexpr int TILE_WORDS = TILE * TILE / 2;
 
-// Row-wise quantisation of a staged tile into q [rows, cols] (+ scales): item = (row, block of 32 columns);
-// consecutive lanes take consecutive rows (conflict-free with the odd pitch).
-__device__ __forceinline__ void quantize_tile_rows(const uint32_t* tile, uint8_t* q, uint8_t* sc, int64_t row_base,
-                                                   int64_t r0, int64_t c0, int64_t cols) {
-    for (int item = threadIdx.x; item < TILE * 4; item += blockDim.x) {
-        const int r = item & 127, kb = item >> 7;
-        uint32_t w[16];
-        uint32_t m = 0u;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            w[i] = tile[r * WPITCH + kb * 16 + i];
-            m = absmax2(m, w[i]);
-        }
-        float inv;
-        const uint32_t byte = scale_byte(fmaxf(bf16_lo(m), bf16_hi(m)), &inv);
-        uint32_t out[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            out[i] = e4m3x4(bf16_lo(w[2 * i]) * inv, bf16_hi(w[2 * i]) * inv, bf16_lo(w[2 * i + 1]) * inv, bf16_hi(w[2 * i + 1]) * inv);
-        st_global_32B(q + (row_base + r0 + r) * cols + c0 + kb * 32, out);
-        sc[scale_offset(row_base + r0 + r, (c0 >> 5) + kb, cols >> 7)] = static_cast<uint8_t>(byte);
-    }
+// Where word c (a pair of columns) of row r lies in a staged tile: 64 words per row in 16-byte units, the unit number
+// XORed so that both passes are free of bank conflicts.  A row is written by eight lanes, 32 bytes each: flipping the
+// lowest bit in the upper half of the row spreads a quarter-warp's 16-byte stores over all banks.  A warp reads eight
+// words of each of four rows that lie 32 apart: the row's block number, shifted by one, puts those on different banks.
+__device__ __forceinline__ int tile_unit(int r, int u) { return r * 16 + (u ^ (u >> 3) ^ ((r >> 5) << 1)); }
+__device__ __forceinline__ void stage_16_columns(uint32_t* tile, int r, int seg, const uint32_t (&w)[8]) {
+    uint4* t = reinterpret_cast<uint4*>(tile);
+    t[tile_unit(r, 2 * seg)] = make_uint4(w[0], w[1], w[2], w[3]);
+    t[tile_unit(r, 2 * seg + 1)] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
-// Column-wise quantisation into qt [cols, rows] (+ scales): item = (pair of adjacent columns, block of 32 rows);
-// consecutive lanes take consecutive column pairs.
+// Row-wise quantisation from registers: lanes 2j and 2j+1 hold one 32-value block (16 consecutive values each).
+// Eight lanes store 128 contiguous bytes of a row.
+__device__ __forceinline__ void quantize_16_columns(const uint32_t (&w)[8], uint8_t* q_dst, uint8_t* sc_dst) {
+    uint32_t m = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = absmax2(m, w[i]);
+    float amax = fmaxf(bf16_lo(m), bf16_hi(m));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    float inv;
+    const uint32_t byte = scale_byte(amax, &inv);
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        o[i] = e4m3x4(bf16_lo(w[2 * i]) * inv, bf16_hi(w[2 * i]) * inv, bf16_lo(w[2 * i + 1]) * inv, bf16_hi(w[2 * i + 1]) * inv);
+    *reinterpret_cast<uint4*>(q_dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    if ((threadIdx.x & 1) == 0) *sc_dst = static_cast<uint8_t>(byte);
+}
+
+// Column-wise quantisation of a staged tile into qt [cols, rows] (+ scales), 256 threads: a thread owns 32 rows of a pair
+// of adjacent columns.  The four row blocks of a column sit in neighbouring lanes, so that a store instruction writes
+// whole 128-byte lines of eight columns instead of 32 bytes of 32 of them.
 __device__ __forceinline__ void quantize_tile_cols(const uint32_t* tile, uint8_t* qt, uint8_t* sct, int64_t col_base,
                                                    int64_t r0, int64_t c0, int64_t rows) {
-    for (int item = threadIdx.x; item < (TILE / 2) * 4; item += blockDim.x) {
-        const int cp = item & 63, kb = item >> 6;
-        uint32_t w[32];
-        uint32_t m = 0u;
+    const int kb = threadIdx.x & 3, cp = threadIdx.x >> 2;
+    uint32_t w[32];
+    uint32_t m = 0u;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            w[i] = tile[(kb * 32 + i) * WPITCH + cp];
-            m = absmax2(m, w[i]);
-        }
-        float inv_a, inv_b;
-        const uint32_t byte_a = scale_byte(bf16_lo(m), &inv_a);
-        const uint32_t byte_b = scale_byte(bf16_hi(m), &inv_b);
-        uint32_t out[8];
-        const int64_t col = col_base + c0 + 2 * cp;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            out[i] = e4m3x4(bf16_lo(w[4 * i]) * inv_a, bf16_lo(w[4 * i + 1]) * inv_a, bf16_lo(w[4 * i + 2]) * inv_a, bf16_lo(w[4 * i + 3]) * inv_a);
-        st_global_32B(qt + col * rows + r0 + kb * 32, out);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            out[i] = e4m3x4(bf16_hi(w[4 * i]) * inv_b, bf16_hi(w[4 * i + 1]) * inv_b, bf16_hi(w[4 * i + 2]) * inv_b, bf16_hi(w[4 * i + 3]) * inv_b);
-        st_global_32B(qt + (col + 1) * rows + r0 + kb * 32, out);
-        sct[scale_offset(col, (r0 >> 5) + kb, rows >> 7)] = static_cast<uint8_t>(byte_a);
-        sct[scale_offset(col + 1, (r0 >> 5) + kb, rows >> 7)] = static_cast<uint8_t>(byte_b);
+    for (int i = 0; i < 32; ++i) {
+        w[i] = tile[tile_unit(kb * 32 + i, cp >> 2) * 4 + (cp & 3)];
+        m = absmax2(m, w[i]);
     }
-}
-
-// 128 x 128 bf16 from global memory (row stride ld elements) into a staged tile, 32 bytes per thread per load
-__device__ __forceinline__ void load_tile_bf16(uint32_t* tile, const __nv_bfloat16* src, int64_t ld) {
-    // 1024 chunks of 32 bytes over 256 threads: all four loads are issued before the first store
-    uint32_t val[4][8];
+    float inv_a, inv_b;
+    const uint32_t byte_a = scale_byte(bf16_lo(m), &inv_a);
+    const uint32_t byte_b = scale_byte(bf16_hi(m), &inv_b);
+    uint32_t out[8];
+    const int64_t col = col_base + c0 + 2 * cp;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int i = threadIdx.x + 256 * k;
-        ld_global_32B(src + static_cast<int64_t>(i >> 3) * ld + (i & 7) * 16, val[k]);
-    }
+    for (int i = 0; i < 8; ++i)
+        out[i] = e4m3x4(bf16_lo(w[4 * i]) * inv_a, bf16_lo(w[4 * i + 1]) * inv_a, bf16_lo(w[4 * i + 2]) * inv_a, bf16_lo(w[4 * i + 3]) * inv_a);
+    st_global_32B(qt + col * rows + r0 + kb * 32, out);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int i = threadIdx.x + 256 * k;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) tile[(i >> 3) * WPITCH + (i & 7) * 8 + j] = val[k][j];
-    }
+    for (int i = 0; i < 8; ++i)
+        out[i] = e4m3x4(bf16_hi(w[4 * i]) * inv_b, bf16_hi(w[4 * i + 1]) * inv_b, bf16_hi(w[4 * i + 2]) * inv_b, bf16_hi(w[4 * i + 3]) * inv_b);
+    st_global_32B(qt + (col + 1) * rows + r0 + kb * 32, out);
+    sct[scale_offset(col, (r0 >> 5) + kb, rows >> 7)] = static_cast<uint8_t>(byte_a);
+    sct[scale_offset(col + 1, (r0 >> 5) + kb, rows >> 7)] = static_cast<uint8_t>(byte_b);
 }
 
 // Rows [begin, min(end, *num_rows)); the grid's y index counts 128-row tiles from `begin`.  Row numbers are those of the
@@ -113,7 +100,7 @@ __global__ void __launch_bounds__(256) quantize_kernel(const __nv_bfloat16* __re
                                                        RowWindow win,
                                                        uint8_t* __restrict__ q, uint8_t* __restrict__ sc,
                                                        uint8_t* __restrict__ qt, uint8_t* __restrict__ sct, int32_t* done_counter) {
-    __shared__ uint32_t tile[TILE_WORDS];
+    __shared__ __align__(16) uint32_t tile[TILE_WORDS];
     const int live = win.num_rows ? min(max(*win.num_rows, 0), win.end) : win.end;
     const int64_t row_tiles = live > win.begin ? (live - win.begin + TILE - 1) / TILE : 0;
     const int64_t col_tiles = N / TILE;
@@ -124,9 +111,18 @@ __global__ void __launch_bounds__(256) quantize_kernel(const __nv_bfloat16* __re
         const int64_t rt = rem / col_tiles;
         const int64_t c0 = (rem - rt * col_tiles) * TILE;
         const int64_t r0 = win.begin + rt * TILE;
-        load_tile_bf16(tile, x + (e * M + r0) * N + c0, N);
+        const int seg = threadIdx.x & 7, rr = threadIdx.x >> 3;      // 16 columns of rows rr, rr + 32, ..
+        const __nv_bfloat16* src = x + (e * M + r0 + rr) * N + c0 + seg * 16;
+        uint32_t val[4][8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ld_global_32B(src + 32 * k * N, val[k]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int64_t row = e * M + r0 + rr + 32 * k;
+            if (qt) stage_16_columns(tile, rr + 32 * k, seg, val[k]);
+            if (q) quantize_16_columns(val[k], q + row * N + c0 + seg * 16, sc + scale_offset(row, (c0 >> 5) + (seg >> 1), N >> 7));
+        }
         __syncthreads();
-        if (q) quantize_tile_rows(tile, q, sc, e * M, r0, c0, N);
         if (qt) quantize_tile_cols(tile, qt, sct, e * N, r0, c0, M);
         __syncthreads();          // the tile is free for the next load
     }
@@ -208,63 +204,59 @@ __device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t v) {
     return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
 
-// Row-wise quantisation of one whole 32-element block: 16 packed words in shared memory.
-__device__ __forceinline__ void quantize_block_smem(const uint32_t* src, uint8_t* q_dst, uint8_t* sc_dst) {
-    uint32_t w[16];
-    uint32_t m = 0u;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        w[j] = src[j];
-        m = absmax2(m, w[j]);
-    }
-    float inv;
-    const uint32_t byte = scale_byte(fmaxf(bf16_lo(m), bf16_hi(m)), &inv);
-    uint32_t out[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        out[j] = e4m3x4(bf16_lo(w[2 * j]) * inv, bf16_hi(w[2 * j]) * inv, bf16_lo(w[2 * j + 1]) * inv, bf16_hi(w[2 * j + 1]) * inv);
-    st_global_32B(q_dst, out);
-    *sc_dst = static_cast<uint8_t>(byte);
-}
-
 // Saved gate/up (E4M3 + scales), d_hidden bf16 -> d_gate, d_up, their row-wise and column-wise quantisations,
 // and the per-(row, 128-column block) router-gradient partial sum(d_hidden * silu(g) * u) / w.
-// grid (I/128, window rows/128), 256 threads: two threads per row, 64 columns (two scale blocks) each, columns in
-// ascending order.  d_gate / d_up are quantised row-wise from registers and staged (two tiles) for the column-wise pass.
+// grid (I/128, window rows/128), 256 threads: eight threads per row, 16 columns each, rows 32 apart in four trips; the next
+// trip's operands are in flight while this one's are worked on.  Every global access of a warp covers whole 128-byte
+// lines of four rows.  d_gate / d_up are quantised row-wise from registers and staged (two tiles) for the column-wise pass.
 __global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
     const uint8_t* __restrict__ gate_q, const uint8_t* __restrict__ gate_sc, const uint8_t* __restrict__ up_q,
     const uint8_t* __restrict__ up_sc, const __nv_bfloat16* __restrict__ d_hidden, int64_t rows_cap, int64_t I,
     RowWindow win, Clamp c, const float* __restrict__ row_scale,
     uint8_t* dg_q, uint8_t* dg_sc, uint8_t* dg_qt, uint8_t* dg_sct,
     uint8_t* du_q, uint8_t* du_sc, uint8_t* du_qt, uint8_t* du_sct, float* __restrict__ partials) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     uint32_t *tdg = sm, *tdu = sm + TILE_WORDS;
-    __shared__ float row_part[TILE][2];
     const int64_t c0 = static_cast<int64_t>(blockIdx.x) * TILE;
     int64_t r0;
     if (!tile_in_window(win, &r0)) return;
-    const int r = threadIdx.x & 127, half = threadIdx.x >> 7;
-    const int64_t row = r0 + r;
-    const float w = row_scale ? row_scale[row] : 1.0f;
-    const float inv_w = w > 0.0f ? 1.0f / w : 0.0f;
-    float partial = 0.0f;
+    const int seg = threadIdx.x & 7, rr = threadIdx.x >> 3;
+    const int64_t col = c0 + seg * 16;
+    const size_t sc_off = scale_offset(r0 + rr, col >> 5, I >> 7);      // of row rr + 32 k: 4 k bytes further on
+    struct Operands {
+        uint4 g, u;
+        uint32_t dh[8];
+        uint32_t gs, us;
+        float w;
+    };
+    auto fetch = [&](int k) {
+        Operands o;
+        const int64_t row = r0 + rr + 32 * k;
+        o.g = *reinterpret_cast<const uint4*>(gate_q + row * I + col);
+        o.u = *reinterpret_cast<const uint4*>(up_q + row * I + col);
+        ld_global_32B(d_hidden + row * I + col, o.dh);
+        o.gs = gate_sc[sc_off + 4 * k];
+        o.us = up_sc[sc_off + 4 * k];
+        o.w = row_scale ? row_scale[row] : 1.0f;
+        return o;
+    };
+    Operands next = fetch(0);
 #pragma unroll 1
-    for (int kb = half * 2; kb < half * 2 + 2; ++kb) {
-        const int64_t col = c0 + kb * 32;
-        const size_t sc_off = scale_offset(row, col >> 5, I >> 7);
-        const float gs = __uint_as_float(static_cast<uint32_t>(gate_sc[sc_off]) << 23);
-        const float us = __uint_as_float(static_cast<uint32_t>(up_sc[sc_off]) << 23);
-        uint32_t gv[8], uv[8], dh[16];
-        ld_global_32B(gate_q + row * I + col, gv);
-        ld_global_32B(up_q + row * I + col, uv);
-        ld_global_32B(d_hidden + row * I + col, reinterpret_cast<uint32_t (&)[8]>(dh[0]));
-        ld_global_32B(d_hidden + row * I + col + 16, reinterpret_cast<uint32_t (&)[8]>(dh[8]));
+    for (int k = 0; k < 4; ++k) {
+        const Operands o = next;
+        if (k < 3) next = fetch(k + 1);
+        const int64_t row = r0 + rr + 32 * k;
+        const float gs = __uint_as_float(o.gs << 23), us = __uint_as_float(o.us << 23);
+        const float inv_w = o.w > 0.0f ? 1.0f / o.w : 0.0f;
+        const uint32_t gv[4] = {o.g.x, o.g.y, o.g.z, o.g.w}, uv[4] = {o.u.x, o.u.y, o.u.z, o.u.w};
+        uint32_t wg[8], wu[8];
+        float partial = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
+        for (int i = 0; i < 8; ++i) {
             const float2 gq = e4m3x2_to_float2(gv[i >> 1] >> ((i & 1) * 16));
             const float2 uq = e4m3x2_to_float2(uv[i >> 1] >> ((i & 1) * 16));
             const float gg[2] = {gq.x * gs, gq.y * gs}, uu[2] = {uq.x * us, uq.y * us};
-            const float dhv[2] = {bf16_lo(dh[i]), bf16_hi(dh[i])};
+            const float dhv[2] = {bf16_lo(o.dh[i]), bf16_hi(o.dh[i])};
             float dg[2], du[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -283,16 +275,20 @@ __global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
                 du[j] = u_ok ? silu * dhv[j] : 0.0f;
                 partial += dhv[j] * inv_w * (silu * u);
             }
-            tdg[r * WPITCH + kb * 16 + i] = pack2(dg[0], dg[1]);
-            tdu[r * WPITCH + kb * 16 + i] = pack2(du[0], du[1]);
+            wg[i] = pack2(dg[0], dg[1]);
+            wu[i] = pack2(du[0], du[1]);
         }
-        // row-wise pass on the words this thread has just staged (its own: no barrier needed)
-        quantize_block_smem(tdg + r * WPITCH + kb * 16, dg_q + row * I + col, dg_sc + sc_off);
-        quantize_block_smem(tdu + r * WPITCH + kb * 16, du_q + row * I + col, du_sc + sc_off);
+        stage_16_columns(tdg, rr + 32 * k, seg, wg);
+        stage_16_columns(tdu, rr + 32 * k, seg, wu);
+        quantize_16_columns(wg, dg_q + row * I + col, dg_sc + sc_off + 4 * k);
+        quantize_16_columns(wu, du_q + row * I + col, du_sc + sc_off + 4 * k);
+        if (partials) {
+#pragma unroll
+            for (int d = 4; d >= 1; d >>= 1) partial += __shfl_xor_sync(0xffffffffu, partial, d);
+            if (seg == 0) partials[row * (I >> 7) + blockIdx.x] = partial;
+        }
     }
-    row_part[r][half] = partial;
     __syncthreads();
-    if (partials && half == 0) partials[row * (I >> 7) + blockIdx.x] = row_part[r][0] + row_part[r][1];
     quantize_tile_cols(tdg, dg_qt, dg_sct, 0, r0, c0, rows_cap);
     quantize_tile_cols(tdu, du_qt, du_sct, 0, r0, c0, rows_cap);
 }
