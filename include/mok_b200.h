@@ -103,7 +103,7 @@ int mokb_schedule(const int32_t* topk_all, int ep_size, int num_local_tokens, in
  * owns the device heap through its own pool, a step loop where cudaMalloc's implicit
  * synchronisation is unaffordable, a process that commits all its memory at start-up:
  * same inputs, outputs and result as mokb_schedule, but the work area is a fixed array
- * inside the library image (4 MiB + 16 KiB, resident on every GPU that loads the library,
+ * inside the library image (512 KiB, resident on every GPU that loads the library,
  * until the process exits) instead of caller-provided scratch.  The caller still passes all
  * inputs and outputs.  The call makes no cudaMalloc / cudaFree and uses no allocating routine.
  *   - Limit: ep_size * num_local_experts <= MOKB_SCHEDULE_NOALLOC_MAX_EXPERTS; beyond it the

@@ -70,20 +70,31 @@ __global__ void prologue_kernel(const int32_t* __restrict__ tokens_per_expert, c
                                 const int32_t* __restrict__ peer_rank, int E_l, int capacity, int MB, int T, Scratch s, int32_t* status) {
     __shared__ int32_t offs[2049];
     __shared__ int32_t ok_s;
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int e = 0; e < E_l; ++e) {
-            offs[e] = run;
-            run += tokens_per_expert[e];
+    for (int e = threadIdx.x; e < E_l; e += blockDim.x) offs[e + 1] = tokens_per_expert[e];
+    const int n = threadIdx.x == 0 ? *num_tokens : 0;
+    __syncthreads();
+    if (threadIdx.x < 32) {          // inclusive scan in place, 32 experts at a time
+        int carry = 0;
+        for (int e0 = 0; e0 < E_l; e0 += 32) {
+            const int e = e0 + static_cast<int>(threadIdx.x);
+            int inc = e < E_l ? offs[e + 1] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (threadIdx.x >= o) inc += v;
+            }
+            if (e < E_l) offs[e + 1] = carry + inc;
+            carry += __shfl_sync(0xffffffffu, inc, 31);
         }
-        offs[E_l] = run;
-        const int n = *num_tokens;
-        int ok = 1;
-        if (n != run || n < 0 || n > capacity) { ok = 0; atomicCAS(status, MOKB_ST_OK, MOKB_ST_SCHEDULE_OVERFLOW); }
-        ok_s = ok;
-        *s.n_rows = ok ? n : 0;
-        s.shared_offsets[0] = 0;
-        s.shared_offsets[1] = T;
+        if (threadIdx.x == 0) {
+            offs[0] = 0;
+            int ok = 1;
+            if (n != carry || n < 0 || n > capacity) { ok = 0; atomicCAS(status, MOKB_ST_OK, MOKB_ST_SCHEDULE_OVERFLOW); }
+            ok_s = ok;
+            *s.n_rows = ok ? n : 0;
+            s.shared_offsets[0] = 0;
+            s.shared_offsets[1] = T;
+        }
     }
     __syncthreads();
     const int ok = ok_s;
@@ -96,10 +107,15 @@ __global__ void prologue_kernel(const int32_t* __restrict__ tokens_per_expert, c
         int end = ok ? offs[e + 1] : 0;
         const int begin = ok ? offs[e] : 0;
         if (end > begin) {
-            int lo = end - 256, hi = end;          // first row in [lo, hi) with peer_rank < 0, or hi
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (peer_rank[mid] < 0) hi = mid; else lo = mid + 1;
+            // sixteen probes at a time: two round trips to memory (a binary search takes eight).  The second round covers
+            // the sixteen rows from the last scheduled probe of the first on.
+            int lo = max(end - 256, begin);
+#pragma unroll
+            for (int step = 16; step >= 1; step /= 16) {
+                int real = 0;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) real += (lo + i * step < end && peer_rank[lo + i * step] >= 0) ? 1 : 0;
+                lo += step > 1 ? max(real - 1, 0) * step : real;
             }
             end = lo;
         }
@@ -134,7 +150,7 @@ __global__ void prologue_kernel(const int32_t* __restrict__ tokens_per_expert, c
 inline int run_prologue(const int32_t* tpe, const int32_t* num_tokens, const int32_t* peer_rank, int E_l, int C, int MB, int T, const Scratch& s,
                         int32_t* status, cudaStream_t stream) {
     MOKB_REQUIRE(E_l <= 2048, "layer: at most 2048 local experts");
-    prologue_kernel<<<1, 256, 0, stream>>>(tpe, num_tokens, peer_rank, E_l, C, MB, T, s, status);
+    prologue_kernel<<<1, 1024, 0, stream>>>(tpe, num_tokens, peer_rank, E_l, C, MB, T, s, status);
     MOKB_CUDA(cudaGetLastError());
     note_launch();
     return MOKB_OK;

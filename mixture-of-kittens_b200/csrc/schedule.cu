@@ -7,18 +7,20 @@
 // strides over that rank's route list (thread index first, then iteration).
 //
 // The reference launches E_l*R blocks that each re-read one rank's whole route
-// list twice.  Here every route is read twice in total:
+// list twice.  Here two launches of about 128 blocks do it:
 //   view a rank's routes as a matrix [iteration][1024 threads]; the reference
-//   order is column-major over that matrix.  A column is split into RC row
-//   chunks, giving V = 1024*RC "virtual columns" in order.
-//   1. count   : one thread per virtual column histograms its routes by local
-//                expert in shared memory -> colcnt[r][e][v]; block sums go to
-//                cnt[e][r] with integer atomics.
-//   2. finalize: tokens_per_expert, segment bases, num_tokens, overflow check.
-//   3. scan    : exclusive scan of colcnt[r][e][:] over v (one block per row).
-//   4. place   : same walk as 1 with the counters started at the scanned
-//                prefix, so each route knows its j and computes its row with
-//                the closed form of scheduler.cuh:134-139.
+//   order is column-major over that matrix.  A block owns a contiguous range of
+//   columns, i.e. a contiguous range of the order.
+//   1. count : every block histograms its routes by local expert.
+//   2. place : every block adds up all blocks' histograms (totals per rank and
+//              expert, and what the blocks before it hold), scans the padded
+//              totals into segment bases, ranks its routes -- a warp takes 32 in
+//              order at a time, lanes of the same expert are ranked by a vote --
+//              and writes each one's row with the closed form of
+//              scheduler.cuh:134-139.  Rows without a route are written by the
+//              same launch, so nothing is cleared beforehand.
+// Bound by latency (about 1 MB moves): what counts is the number of dependent launches and
+// round trips.  Earlier: three clears and four kernels.
 #include "common.cuh"
 
 namespace mokb {
@@ -26,17 +28,16 @@ namespace {
 
 constexpr int kThreadsOrder = 1024;   // the reference's block size, which defines the order
 constexpr int kPad = 256;             // expert segment padding
+constexpr int kSchedThreads = 512;
+constexpr int kSchedWarps = kSchedThreads / 32;
+constexpr int kMaxColumnBlocks = 128;
 
 struct SchedParams {
     const int32_t* topk_all;  // [R, routes]
     int R, routes, E_l, C, rank;
-    int RC;                   // row chunks per column
-    int rows_per_chunk;       // ceil(ceil(routes/1024) / RC)
-    int V;                    // 1024 * RC
-    int32_t* cnt;             // [E_l, R]
-    int32_t* base;            // [E_l + 1]
-    int32_t* overflow;        // [1]
-    int32_t* colcnt;          // [R, E_l, V]
+    int NB;                   // blocks per rank: a power of two; each owns 1024 / NB columns
+    int P;                    // ceil(routes / 1024): rows of the matrix
+    int32_t* blkcnt;          // [R, NB, E_l]
     int32_t* peer_rank;
     int32_t* peer_token_idx;
     int32_t* num_tokens;
@@ -44,137 +45,161 @@ struct SchedParams {
     int32_t* status;
 };
 
-template <bool PLACE>
-__global__ void walk_kernel(SchedParams p) {
-    extern __shared__ int32_t sm[];
-    const int cpb = blockDim.x;
-    int32_t* counters = sm;                         // [E_l][cpb]
-    int32_t* cnt_s = counters + p.E_l * cpb;        // [E_l][R]   (PLACE)
-    int32_t* base_s = cnt_s + p.E_l * p.R;          // [E_l]      (PLACE)
-    const int r = blockIdx.y;
-    const int v0 = blockIdx.x * cpb;
-    const int t = threadIdx.x;
-    const int v = v0 + t;
+__global__ void __launch_bounds__(kSchedThreads) count_kernel(SchedParams p) {
+    extern __shared__ int32_t hist[];     // [E_l]
+    const int t = threadIdx.x, r = blockIdx.y, b = blockIdx.x;
+    for (int e = t; e < p.E_l; e += kSchedThreads) hist[e] = 0;
+    __syncthreads();
+    const uint32_t cols = kThreadsOrder / p.NB, c0 = b * cols, shift = 31 - __clz(cols);
     const int first = p.rank * p.E_l;
-
-    if (PLACE) {
-        if (*p.overflow) return;
-        for (int i = t; i < p.E_l * p.R; i += cpb) cnt_s[i] = p.cnt[i];
-        for (int i = t; i < p.E_l; i += cpb) base_s[i] = p.base[i];
-        for (int e = 0; e < p.E_l; ++e)
-            counters[e * cpb + t] = p.colcnt[(static_cast<size_t>(r) * p.E_l + e) * p.V + v];
-    } else {
-        for (int e = 0; e < p.E_l; ++e) counters[e * cpb + t] = 0;
+    const int32_t* routes = p.topk_all + static_cast<size_t>(r) * p.routes;
+    const uint32_t items = p.P * cols;           // any order will do here: row by row
+#pragma unroll 4
+    for (uint32_t i = t; i < items; i += kSchedThreads) {
+        const uint32_t idx = (i >> shift) * kThreadsOrder + c0 + (i & (cols - 1));
+        if (idx < static_cast<uint32_t>(p.routes)) {
+            const int e = __ldg(routes + idx) - first;
+            if (e >= 0 && e < p.E_l) atomicAdd(&hist[e], 1);
+        }
     }
     __syncthreads();
+    int32_t* out = p.blkcnt + (static_cast<size_t>(r) * p.NB + b) * p.E_l;
+    for (int e = t; e < p.E_l; e += kSchedThreads) out[e] = hist[e];
+}
 
-    const int32_t* routes = p.topk_all + static_cast<size_t>(r) * p.routes;
-    const int c = v / p.RC, q = v - c * p.RC;
-    const int row0 = q * p.rows_per_chunk;
-    constexpr int U = 8;
-    for (int s0 = 0; s0 < p.rows_per_chunk; s0 += U) {
-        int idx[U], ex[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int s = s0 + u;
-            const int i = (row0 + s) * kThreadsOrder + c;
-            idx[u] = (s < p.rows_per_chunk && i < p.routes) ? i : -1;
-            ex[u] = idx[u] >= 0 ? __ldg(routes + idx[u]) - first : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int e = ex[u];
-            if (idx[u] >= 0 && e >= 0 && e < p.E_l) {
-                const int j = counters[e * cpb + t]++;
-                if (PLACE) {
-                    int dst = base_s[e];
-                    const int32_t* ce = cnt_s + e * p.R;
-                    for (int rr = 0; rr < p.R; ++rr) {
-                        const int n = ce[rr];
-                        dst += min(n, j) + ((rr < r && n > j) ? 1 : 0);
-                    }
-                    p.peer_rank[dst] = r;
-                    p.peer_token_idx[dst] = idx[u];
-                }
+__global__ void __launch_bounds__(kSchedThreads) place_kernel(SchedParams p) {
+    extern __shared__ int32_t sm[];
+    int32_t* const tot = sm;                              // [R][E_l]  routes of a rank to an expert
+    int32_t* const ctr = tot + p.R * p.E_l;               // [warps][E_l]
+    int32_t* const before = ctr + kSchedWarps * p.E_l;    // [E_l]     routes of this rank in the blocks before this one
+    int32_t* const base = before + p.E_l;                 // [E_l + 1] first row of a segment
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, r = blockIdx.y, b = blockIdx.x;
+    const int E_l = p.E_l, first = p.rank * E_l;
+    for (int i = t; i < (p.R + kSchedWarps + 1) * E_l; i += kSchedThreads) sm[i] = 0;
+    __syncthreads();
+
+    for (int rr = 0; rr < p.R; ++rr) {
+        const int32_t* c = p.blkcnt + static_cast<size_t>(rr) * p.NB * E_l;
+        const int n = p.NB * E_l, mine = rr == r ? b * E_l : 0;     // entries below `mine`: earlier blocks of this rank
+#pragma unroll 4
+        for (int i = t; i < n; i += kSchedThreads) {
+            const int v = __ldg(c + i);
+            if (v) {
+                const int e = i % E_l;
+                atomicAdd(&tot[rr * E_l + e], v);
+                if (i < mine) atomicAdd(&before[e], v);
             }
         }
     }
-    if (PLACE) return;
-    __syncthreads();
-    for (int e = 0; e < p.E_l; ++e)
-        p.colcnt[(static_cast<size_t>(r) * p.E_l + e) * p.V + v] = counters[e * cpb + t];
-    // block total per expert -> cnt[e][r]
-    const int warp = t >> 5, lane = t & 31, nwarps = cpb >> 5;
-    for (int e = warp; e < p.E_l; e += nwarps) {
-        int s = 0;
-        for (int k = lane; k < cpb; k += 32) s += counters[e * cpb + k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0 && s) atomicAdd(&p.cnt[e * p.R + r], s);
+    // this block's part of the order, a contiguous piece of it per warp
+    const uint32_t cols = kThreadsOrder / p.NB, c0 = b * cols, P = p.P;
+    const int32_t* routes = p.topk_all + static_cast<size_t>(r) * p.routes;
+    const uint32_t items = P * cols;             // at most routes + 1023 * cols, routes < 2^31
+    const uint32_t per_warp = (items + kSchedThreads - 1) / kSchedThreads * 32;
+    const uint32_t l0 = warp * per_warp, l1 = min(l0 + per_warp, items);
+    auto expert_of = [&](uint32_t l, int* index) {          // position in the order -> local expert, or -1
+        const uint32_t cc = l / P;
+        const uint32_t idx = (l - cc * P) * kThreadsOrder + c0 + cc;
+        *index = static_cast<int>(idx);
+        if (l >= l1 || idx >= static_cast<uint32_t>(p.routes)) return -1;
+        const int e = __ldg(routes + idx) - first;
+        return e >= 0 && e < E_l ? e : -1;
+    };
+    int index;
+    for (uint32_t l = l0 + lane; l < l1; l += 32) {
+        const int e = expert_of(l, &index);
+        if (e >= 0) atomicAdd(&ctr[warp * E_l + e], 1);
     }
-}
+    __syncthreads();
 
-__device__ __forceinline__ int block_exclusive_scan_1024(int x, int32_t* warp_sums, int* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int inc = x;
+    if (warp == 0) {          // segment bases: exclusive scan of the padded totals
+        int carry = 0;
+        for (int e0 = 0; e0 < E_l; e0 += 32) {
+            const int e = e0 + lane;
+            int padded = 0;
+            if (e < E_l) {
+                int n = 0;
+                for (int rr = 0; rr < p.R; ++rr) n += tot[rr * E_l + e];
+                padded = (n + kPad - 1) / kPad * kPad;
+                if (b == 0 && r == 0) p.tokens_per_expert[e] = padded;
+            }
+            int inc = padded;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += n;
-    }
-    if (lane == 31) warp_sums[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        int w = warp_sums[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int n = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += n;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            if (e < E_l) base[e] = carry + inc - padded;
+            carry += __shfl_sync(0xffffffffu, inc, 31);
         }
-        warp_sums[lane] = w;
-    }
-    __syncthreads();
-    const int before = warp ? warp_sums[warp - 1] : 0;
-    if (total) *total = warp_sums[31];
-    __syncthreads();
-    return before + inc - x;
-}
-
-__global__ void finalize_kernel(SchedParams p) {
-    __shared__ int32_t warp_sums[32];
-    int carry = 0;
-    for (int e0 = 0; e0 < p.E_l; e0 += 1024) {
-        const int e = e0 + threadIdx.x;
-        int padded = 0;
-        if (e < p.E_l) {
-            int n = 0;
-            for (int r = 0; r < p.R; ++r) n += p.cnt[e * p.R + r];
-            padded = (n + kPad - 1) / kPad * kPad;
-            p.tokens_per_expert[e] = padded;
+        if (lane == 0) {
+            base[E_l] = carry;
+            if (b == 0 && r == 0) {
+                p.num_tokens[0] = carry;
+                if (carry > p.C) atomicCAS(p.status, MOKB_ST_OK, MOKB_ST_SCHEDULE_OVERFLOW);
+            }
         }
-        int total;
-        const int ex = block_exclusive_scan_1024(padded, warp_sums, &total);
-        if (e < p.E_l) p.base[e] = carry + ex;
-        carry += total;
+    } else {                  // where each warp's routes of an expert start counting
+        for (int e = t - 32; e < E_l; e += kSchedThreads - 32) {
+            int run = before[e];
+            for (int w = 0; w < kSchedWarps; ++w) {
+                const int n = ctr[w * E_l + e];
+                ctr[w * E_l + e] = run;
+                run += n;
+            }
+        }
     }
-    if (threadIdx.x == 0) {
-        p.base[p.E_l] = carry;
-        p.num_tokens[0] = carry;
-        const int over = carry > p.C;
-        *p.overflow = over;
-        if (over) atomicCAS(p.status, MOKB_ST_OK, MOKB_ST_SCHEDULE_OVERFLOW);
+    __syncthreads();
+
+    // rows without a route: all of them if the schedule does not fit, otherwise the end of every segment and of the arrays
+    const int total = base[E_l];
+    const bool overflow = total > p.C;
+    const int block = r * p.NB + b, nblocks = p.NB * p.R;
+    for (int64_t i = (overflow ? 0 : total) + static_cast<int64_t>(block) * kSchedThreads + t; i < p.C; i += static_cast<int64_t>(nblocks) * kSchedThreads)
+        p.peer_rank[i] = p.peer_token_idx[i] = -1;
+    if (overflow) return;
+    for (int e = block * kSchedWarps + warp; e < E_l; e += nblocks * kSchedWarps) {
+        int n = 0;
+        for (int rr = 0; rr < p.R; ++rr) n += tot[rr * E_l + e];
+        for (int i = base[e] + n + lane; i < base[e + 1]; i += 32) p.peer_rank[i] = p.peer_token_idx[i] = -1;
+    }
+
+    int32_t* const count = ctr + warp * E_l;
+    for (uint32_t lb = l0; lb < l1; lb += 32) {            // whole warp: the same number of trips in every lane
+        const int e = expert_of(lb + lane, &index);
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        int j = 0;
+        if (e >= 0) j = count[e] + __popc(same & ((1u << lane) - 1u));
+        __syncwarp();
+        if (e >= 0 && lane == 31 - __clz(same)) count[e] = j + 1;
+        __syncwarp();
+        if (e >= 0) {
+            int dst = base[e];
+            for (int rr = 0; rr < p.R; ++rr) {
+                const int n = tot[rr * E_l + e];
+                dst += min(n, j) + ((rr < r && n > j) ? 1 : 0);
+            }
+            p.peer_rank[dst] = r;
+            p.peer_token_idx[dst] = index;
+        }
     }
 }
 
-__global__ void scan_kernel(SchedParams p) {
-    __shared__ int32_t warp_sums[32];
-    int32_t* row = p.colcnt + static_cast<size_t>(blockIdx.x) * p.V;
-    const int RC = p.RC;
-    int local[8];
-    int sum = 0;
-    for (int k = 0; k < RC; ++k) { local[k] = row[threadIdx.x * RC + k]; sum += local[k]; }
-    int run = block_exclusive_scan_1024(sum, warp_sums, nullptr);
-    for (int k = 0; k < RC; ++k) { row[threadIdx.x * RC + k] = run; run += local[k]; }
+// Blocks: about 128 over all ranks, fewer where the histograms that every block of the second launch adds up would
+// otherwise exceed 16384 words (32 per thread).
+int launch_schedule(SchedParams p, cudaStream_t stream) {
+    const int E = p.R * p.E_l;
+    p.P = (p.routes + kThreadsOrder - 1) / kThreadsOrder;
+    p.NB = kMaxColumnBlocks;
+    while (p.NB > 1 && (p.NB * p.R > kMaxColumnBlocks || static_cast<int64_t>(p.NB) * E > 16384)) p.NB /= 2;
+    const size_t smem = (static_cast<size_t>(E) + static_cast<size_t>(kSchedWarps + 2) * p.E_l + 1) * 4;
+    if (smem > 48 * 1024) MOKB_CUDA(cudaFuncSetAttribute(place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    const dim3 grid(static_cast<unsigned>(p.NB), static_cast<unsigned>(p.R));
+    count_kernel<<<grid, kSchedThreads, static_cast<size_t>(p.E_l) * 4, stream>>>(p);
+    place_kernel<<<grid, kSchedThreads, smem, stream>>>(p);
+    MOKB_CUDA(cudaGetLastError());
+    note_launch(2);
+    return MOKB_OK;
 }
 
 }  // namespace
@@ -182,23 +207,9 @@ __global__ void scan_kernel(SchedParams p) {
 
 using namespace mokb;
 
-static void sched_geometry(int R, int routes, int E_l, int* RC, int* rows_per_chunk, int* cpb) {
-    const int P = (routes + kThreadsOrder - 1) / kThreadsOrder;
-    int rc = 1;
-    while (rc < 8 && R * kThreadsOrder * rc < 16384 && P / (rc * 2) >= 8) rc *= 2;
-    *RC = rc;
-    *rows_per_chunk = (P + rc - 1) / rc;
-    int c = 128;
-    while (c > 32 && static_cast<size_t>(E_l) * c * 4 > 160 * 1024) c /= 2;
-    *cpb = c;
-}
-
 extern "C" size_t mokb_schedule_scratch_bytes(int ep_size, int num_local_experts) {
-    const size_t E = static_cast<size_t>(ep_size) * num_local_experts;
-    // cnt + base + overflow (rounded up), then colcnt at the largest RC
-    size_t head = (E + num_local_experts + 2) * 4;
-    head = (head + 255) / 256 * 256;
-    return head + E * kThreadsOrder * 8 * 4;
+    // an upper bound with room to spare (the histograms take at most a 64th of it); callers may have been sized by it
+    return static_cast<size_t>(ep_size) * num_local_experts * (kThreadsOrder * 8 + 2) * 4;
 }
 
 extern "C" int mokb_schedule(const int32_t* topk_all, int ep_size, int num_local_tokens, int topk,
@@ -221,35 +232,10 @@ extern "C" int mokb_schedule(const int32_t* topk_all, int ep_size, int num_local
     p.topk_all = topk_all;
     p.R = ep_size; p.routes = static_cast<int>(routes_ll); p.E_l = num_local_experts;
     p.C = schedule_capacity; p.rank = rank;
-    int cpb;
-    sched_geometry(p.R, p.routes, p.E_l, &p.RC, &p.rows_per_chunk, &cpb);
-    p.V = kThreadsOrder * p.RC;
-    const size_t E = static_cast<size_t>(p.R) * p.E_l;
-    int32_t* s = static_cast<int32_t*>(scratch);
-    p.cnt = s;
-    p.base = s + E;
-    p.overflow = p.base + p.E_l + 1;
-    size_t head = (E + p.E_l + 2) * 4;
-    head = (head + 255) / 256 * 256;
-    p.colcnt = reinterpret_cast<int32_t*>(static_cast<char*>(scratch) + head);
+    p.blkcnt = static_cast<int32_t*>(scratch);
     p.peer_rank = peer_rank; p.peer_token_idx = peer_token_idx;
     p.num_tokens = num_tokens; p.tokens_per_expert = tokens_per_expert; p.status = status;
-
-    MOKB_CUDA(cudaMemsetAsync(p.cnt, 0, head, stream));
-    MOKB_CUDA(cudaMemsetAsync(peer_rank, 0xFF, static_cast<size_t>(schedule_capacity) * 4, stream));
-    MOKB_CUDA(cudaMemsetAsync(peer_token_idx, 0xFF, static_cast<size_t>(schedule_capacity) * 4, stream));
-
-    const size_t smem = (static_cast<size_t>(p.E_l) * cpb + E + p.E_l) * 4;
-    MOKB_CUDA(cudaFuncSetAttribute(walk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    MOKB_CUDA(cudaFuncSetAttribute(walk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    const dim3 grid(p.V / cpb, p.R);
-    walk_kernel<false><<<grid, cpb, smem, stream>>>(p);
-    finalize_kernel<<<1, 1024, 0, stream>>>(p);
-    scan_kernel<<<static_cast<unsigned>(E), 1024, 0, stream>>>(p);
-    walk_kernel<true><<<grid, cpb, smem, stream>>>(p);
-    MOKB_CUDA(cudaGetLastError());
-    note_launch(4);
-    return MOKB_OK;
+    return launch_schedule(p, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -265,9 +251,9 @@ extern "C" int mokb_schedule(const int32_t* topk_all, int ep_size, int num_local
 namespace mokb {
 namespace {
 
-constexpr size_t kStaticHeadBytes = 16u << 10;     // cnt[E] + base[E_l + 1] + overflow flag
-constexpr size_t kStaticColcntBytes = 4u << 20;    // colcnt[E][1024 * RC]: E * RC <= 1024
-static __device__ __align__(256) unsigned char g_static_sched_scratch[kStaticHeadBytes + kStaticColcntBytes];
+// the histograms of every block of the first launch, for the most experts that this entry point takes
+constexpr size_t kStaticSchedBytes = static_cast<size_t>(MOKB_SCHEDULE_NOALLOC_MAX_EXPERTS) * kMaxColumnBlocks * 4;
+static __device__ __align__(256) unsigned char g_static_sched_scratch[kStaticSchedBytes];
 
 // Device address of the array above, per device.  In host code the array's name is only a
 // handle for the runtime; the address a kernel can use comes from cudaGetSymbolAddress,
@@ -318,38 +304,9 @@ extern "C" int mokb_schedule_noalloc(const int32_t* topk_all, int ep_size, int n
     p.topk_all = topk_all;
     p.R = ep_size; p.routes = static_cast<int>(routes_ll); p.E_l = num_local_experts;
     p.C = schedule_capacity; p.rank = rank;
-    int cpb;
-    sched_geometry(p.R, p.routes, p.E_l, &p.RC, &p.rows_per_chunk, &cpb);
-    // fewer row chunks per column until colcnt fits the fixed area (the result does not depend on RC)
-    while (p.RC > 1 && E * kThreadsOrder * p.RC * 4 > kStaticColcntBytes) p.RC /= 2;
-    const int P = (p.routes + kThreadsOrder - 1) / kThreadsOrder;
-    p.rows_per_chunk = (P + p.RC - 1) / p.RC;
-    p.V = kThreadsOrder * p.RC;
-    MOKB_REQUIRE(E * p.V * 4 <= kStaticColcntBytes && (E + p.E_l + 2) * 4 <= kStaticHeadBytes,
-                 "schedule_noalloc: problem does not fit the built-in work area");
-    int32_t* s = static_cast<int32_t*>(scratch);
-    p.cnt = s;
-    p.base = s + E;
-    p.overflow = p.base + p.E_l + 1;
-    p.colcnt = reinterpret_cast<int32_t*>(static_cast<char*>(scratch) + kStaticHeadBytes);
+    // the area keeps whatever the previous call left; every word that is read is written by this call's first launch
+    p.blkcnt = static_cast<int32_t*>(scratch);
     p.peer_rank = peer_rank; p.peer_token_idx = peer_token_idx;
     p.num_tokens = num_tokens; p.tokens_per_expert = tokens_per_expert; p.status = status;
-
-    // the area keeps whatever the previous call left: the counters and the overflow flag must start at zero
-    // (colcnt is fully rewritten by the counting pass before anything reads it)
-    MOKB_CUDA(cudaMemsetAsync(scratch, 0, kStaticHeadBytes, stream));
-    MOKB_CUDA(cudaMemsetAsync(peer_rank, 0xFF, static_cast<size_t>(schedule_capacity) * 4, stream));
-    MOKB_CUDA(cudaMemsetAsync(peer_token_idx, 0xFF, static_cast<size_t>(schedule_capacity) * 4, stream));
-
-    const size_t smem = (static_cast<size_t>(p.E_l) * cpb + E + p.E_l) * 4;
-    MOKB_CUDA(cudaFuncSetAttribute(walk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    MOKB_CUDA(cudaFuncSetAttribute(walk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    const dim3 grid(p.V / cpb, p.R);
-    walk_kernel<false><<<grid, cpb, smem, stream>>>(p);
-    finalize_kernel<<<1, 1024, 0, stream>>>(p);
-    scan_kernel<<<static_cast<unsigned>(E), 1024, 0, stream>>>(p);
-    walk_kernel<true><<<grid, cpb, smem, stream>>>(p);
-    MOKB_CUDA(cudaGetLastError());
-    note_launch(4);
-    return MOKB_OK;
+    return launch_schedule(p, stream);
 }
