@@ -220,6 +220,35 @@ __device__ __forceinline__ bool flag_wait(const int* flag, int target, volatile 
     }
 }
 
+// ---- the order of the tiles of a routed forward launch (gate/up + SwiGLU tiles, and down tiles that need all gate/up
+// tiles of their 256 rows).  Super-groups of `gm` row tiles x every column tile, the down tiles `lag` super-groups behind:
+//   gu(0) .. gu(lag)  down(0)  gu(lag + 1)  down(1)  ..        (gu(i) = gate/up tiles of super-group i)
+// A CTA takes every `stride`-th tile of this one order, so a down tile never waits for a tile that comes after it, and with
+// two rounds of tiles between a gate/up tile and the down tiles of its rows (its main loop and its epilogue) it hardly waits at all.
+__device__ __forceinline__ int fwd_lag(int stride, int gm, int n_gu, int n_nt) {
+    const int per = gm * (n_gu + n_nt);
+    return (2 * stride + per - 1) / per;
+}
+// Whether windows are long enough to take all gate/up tiles of a window first and then all its down tiles (which re-reads fewer
+// weights: a gate/up super-group follows the previous one of the same expert directly) without waiting at either end.
+__device__ __forceinline__ bool fwd_by_window(int win_blocks, int stride, int gm, int n_gu, int n_nt) {
+    return static_cast<long long>(win_blocks - gm) * min(n_gu, n_nt) >= 2ll * stride;
+}
+// tile t of the lagged order -> phase (0 gate/up, 1 down) and number x of the tile in its phase's own order
+__device__ __forceinline__ void fwd_lagged_tile(int t, int m_blocks, int gm, int lag, int n_gu, int n_nt, int* phase, int* x) {
+    const int sgs = (m_blocks + gm - 1) / gm;
+    const int head = min(lag * gm, m_blocks) * n_gu;
+    if (t < head) { *phase = 0; *x = t; return; }
+    t -= head;
+    if (sgs <= lag) { *phase = 1; *x = t; return; }
+    const int per = gm * (n_gu + n_nt);
+    const int q = min(t / per, sgs - lag - 1);                   // gu(lag + q), then down(q), and after the last one the remaining down tiles
+    t -= q * per;
+    const int gu = min(gm, m_blocks - (lag + q) * gm) * n_gu;
+    *phase = t < gu ? 0 : 1;
+    *x = t < gu ? (lag + q) * gm * n_gu + t : q * gm * n_nt + (t - gu);
+}
+
 // Routes are numbered [0, limit) on every rank; an index outside (a stale or foreign schedule) must not become an access
 // to a peer's memory: the row is skipped and the status words say where (limit <= 0: unchecked).
 struct IndexGuard {

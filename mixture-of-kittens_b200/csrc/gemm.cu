@@ -26,7 +26,7 @@
 //   MODE_NN      D[rows,N] = A[rows,K] * W[g][K,N] (+ A2 * W2[g])    (input gradients)
 //   MODE_WGRAD   D[g][M,N] = A[rows_g,M]^T * B[rows_g,N]             (weight gradients)
 //   MODE_FWD     MODE_SWIGLU tiles and the MODE_NT (down) tiles of the same rows in ONE persistent launch,
-//                window by window (a window = the rows one dispatch launch pulls): the task loop of the
+//                the down tiles some super-groups of rows behind: the task loop of the
 //                reference's forward megakernel (csrc/megakernel/forward.cuh:146-266) with its global-memory
 //                counters (csrc/megakernel/utils.cuh:1-13), every wait bounded.
 // Expert segments are multiples of 256 rows, so a tile never straddles two experts.
@@ -113,10 +113,10 @@ struct Tile {
 template <int MODE, int NCTA>
 struct Sched {
     int m_blocks, n_blocks, total, m_first;
-    int n_gu, n_nt, win_blocks;      // MODE_FWD: column tiles of the two phases; row tiles per window (all row-tiled modes)
+    int n_gu, n_nt, win_blocks, lag;      // MODE_FWD: column tiles of the two phases; row tiles per window (all row-tiled modes)
     __device__ Sched(const KParams& p) {
         m_first = 0;
-        n_gu = n_nt = 0;
+        n_gu = n_nt = lag = 0;
         win_blocks = 1 << 30;
         constexpr int TM = Geo<NCTA>::TILE_M;
         if (MODE == MODE_WGRAD) {
@@ -138,6 +138,8 @@ struct Sched {
                 n_gu = p.N / 128;
                 n_nt = p.N2 / BN;
                 total = m_blocks * (n_gu + n_nt);
+                const int stride = static_cast<int>(gridDim.x >> 1);
+                lag = fwd_by_window(min(win_blocks, m_blocks), stride, Geo<NCTA>::GROUP_M, n_gu, n_nt) ? 0 : fwd_lag(stride, Geo<NCTA>::GROUP_M, n_gu, n_nt);
             }
         }
     }
@@ -156,26 +158,31 @@ struct Sched {
             if (p.group_k_end) k_end = min(k_end, max(p.group_k_end[ti.group], ti.k_row0));
             ti.k_iters = (k_end - ti.k_row0 + BK - 1) / BK;      // a partial last stage reads rows that are zero
         } else if (MODE == MODE_FWD) {
-            // window by window: all gate/up tiles of the window's rows, then all their down tiles; inside a phase,
-            // super-groups of 1024 rows x every column tile
-            const int wb = min(win_blocks, m_blocks);
-            const int per_win = wb * (n_gu + n_nt);
-            const int n_win = (m_blocks + wb - 1) / wb;
-            const int w = min(t / per_win, n_win - 1);
-            int local = t - w * per_win;
-            const int blk0 = w * wb;
-            const int wc = min(wb, m_blocks - blk0);
-            ti.phase = local >= wc * n_gu ? 1 : 0;
-            if (ti.phase) local -= wc * n_gu;
+            int first_blk = 0, blocks = m_blocks, x;             // the row tiles that x, a tile's number in its phase, counts
+            if (lag > 0) {
+                fwd_lagged_tile(t, m_blocks, GM, lag, n_gu, n_nt, &ti.phase, &x);
+            } else {
+                // window by window: all gate/up tiles of the window's rows, then all their down tiles
+                const int wb = min(win_blocks, m_blocks);
+                const int per_win = wb * (n_gu + n_nt);
+                const int w = min(t / per_win, (m_blocks + wb - 1) / wb - 1);
+                first_blk = w * wb;
+                blocks = min(wb, m_blocks - first_blk);
+                x = t - w * per_win;
+                ti.phase = x >= blocks * n_gu ? 1 : 0;
+                if (ti.phase) x -= blocks * n_gu;
+            }
+            // inside a phase: super-groups of 1024 rows x every column tile
             const int nb = ti.phase ? n_nt : n_gu;
             const int per = GM * nb;
-            const int sg = local / per;
+            const int sg = x / per;
             const int first = sg * GM;
-            const int gsize = min(GM, wc - first);
-            const int in = local - sg * per;
+            const int gsize = min(GM, blocks - first);
+            const int in = x - sg * per;
             ti.n_blk = in / gsize;
-            ti.m_blk = m_first + blk0 + first + (in - ti.n_blk * gsize);
-            ti.window = w;
+            const int blk = first_blk + first + (in - ti.n_blk * gsize);
+            ti.m_blk = m_first + blk;
+            ti.window = blk / win_blocks;
             ti.group = p.group_of_block ? p.group_of_block[ti.m_blk * (TM / 128)] : 0;
             ti.k_row0 = 0;
             ti.k_iters = (ti.phase ? p.K2 : p.K) / BK;
@@ -304,7 +311,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             uint32_t ph = 0;
             bool ok = true;
             const int kh = p.K / BK;
-            int waited_window = -1;
+            unsigned long long arrived = 0;        // windows of which this producer knows that their rows have arrived
             // the next tile's coordinates (integer divisions, loads of the group tables) are worked out while this
             // tile's stages are in flight: with a short contraction the look-up would otherwise stall every tile
             Tile next_ti = {};
@@ -316,9 +323,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (MODE != MODE_WGRAD) {
                     // rows that another kernel (or, for a down tile, other CTAs of this one) is still producing
                     bool fenced = false;
-                    if (p.win_ready && ti.phase == 0 && ti.window > waited_window) {
+                    if (p.win_ready && ti.phase == 0 && (ti.window >= 64 || !(arrived >> ti.window & 1))) {
                         if (!flag_wait(p.win_ready + ti.window, p.win_ready_target, abort_flag, p.status, kWaitWindowReady, ti.window)) { ok = false; break; }
-                        waited_window = ti.window;
+                        if (ti.window < 64) arrived |= 1ull << ti.window;
                         fenced = true;
                     }
                     if (MODE == MODE_FWD && ti.phase == 1) {

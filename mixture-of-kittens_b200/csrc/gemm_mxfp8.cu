@@ -101,10 +101,10 @@ struct Tile {
 template <int MODE>
 struct Sched {
     int m_blocks, n_blocks, total, m_first;
-    int n_gu, n_nt, win_blocks;
+    int n_gu, n_nt, win_blocks, lag;
     __device__ Sched(const FParams& p) {
         m_first = 0;
-        n_gu = n_nt = 0;
+        n_gu = n_nt = lag = 0;
         win_blocks = 1 << 30;
         if (MODE == FMODE_WGRAD) {
             m_blocks = (p.M + TILE_M - 1) / TILE_M;
@@ -125,6 +125,8 @@ struct Sched {
                 n_gu = p.N / 128;
                 n_nt = p.N2 / BN;
                 total = m_blocks * (n_gu + n_nt);
+                const int stride = static_cast<int>(gridDim.x >> 1);
+                lag = fwd_by_window(min(win_blocks, m_blocks), stride, GROUP_M, n_gu, n_nt) ? 0 : fwd_lag(stride, GROUP_M, n_gu, n_nt);
             }
         }
     }
@@ -140,24 +142,31 @@ struct Sched {
             ti.k_tile0 = c0 / BKB - p.k_tile_origin;
             ti.k_iters = (p.group_offsets[ti.group + 1] - c0) / BKB;
         } else if (MODE == FMODE_FWD) {
-            const int wb = min(win_blocks, m_blocks);
-            const int per_win = wb * (n_gu + n_nt);
-            const int n_win = (m_blocks + wb - 1) / wb;
-            const int w = min(t / per_win, n_win - 1);
-            int local = t - w * per_win;
-            const int blk0 = w * wb;
-            const int wc = min(wb, m_blocks - blk0);
-            ti.phase = local >= wc * n_gu ? 1 : 0;
-            if (ti.phase) local -= wc * n_gu;
+            int first_blk = 0, blocks = m_blocks, x;             // the row tiles that x, a tile's number in its phase, counts
+            if (lag > 0) {
+                fwd_lagged_tile(t, m_blocks, GROUP_M, lag, n_gu, n_nt, &ti.phase, &x);
+            } else {
+                // window by window: all gate/up tiles of the window's rows, then all their down tiles
+                const int wb = min(win_blocks, m_blocks);
+                const int per_win = wb * (n_gu + n_nt);
+                const int w = min(t / per_win, (m_blocks + wb - 1) / wb - 1);
+                first_blk = w * wb;
+                blocks = min(wb, m_blocks - first_blk);
+                x = t - w * per_win;
+                ti.phase = x >= blocks * n_gu ? 1 : 0;
+                if (ti.phase) x -= blocks * n_gu;
+            }
+            // inside a phase: super-groups of 1024 rows x every column tile
             const int nb = ti.phase ? n_nt : n_gu;
             const int per = GROUP_M * nb;
-            const int sg = local / per;
+            const int sg = x / per;
             const int first = sg * GROUP_M;
-            const int gsize = min(GROUP_M, wc - first);
-            const int in = local - sg * per;
+            const int gsize = min(GROUP_M, blocks - first);
+            const int in = x - sg * per;
             ti.n_blk = in / gsize;
-            ti.m_blk = m_first + blk0 + first + (in - ti.n_blk * gsize);
-            ti.window = w;
+            const int blk = first_blk + first + (in - ti.n_blk * gsize);
+            ti.m_blk = m_first + blk;
+            ti.window = blk / win_blocks;
             ti.group = p.group_of_block ? p.group_of_block[ti.m_blk * 2] : 0;
             ti.k_tile0 = 0;
             ti.k_iters = (ti.phase ? p.K2 : p.K) / BKB;
@@ -277,7 +286,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
             uint32_t ph = 0;
             bool ok = true;
             const int kh = p.K / BKB;
-            int waited_window = -1;
+            unsigned long long arrived = 0;        // windows of which this producer knows that their rows have arrived
             Tile next_ti = {};         // worked out one tile ahead: the look-up would otherwise stall short tiles
             if (tile_id0 < sched.total) next_ti = sched.get(p, tile_id0);
             for (int t = tile_id0; ok && t < sched.total; t += tile_stride) {
@@ -287,9 +296,9 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
                 if (MODE != FMODE_WGRAD) {
                     // rows that another kernel (or, for a down tile, other CTAs of this one) is still producing
                     bool fenced = false;
-                    if (p.win_ready && ti.phase == 0 && ti.window > waited_window) {
+                    if (p.win_ready && ti.phase == 0 && (ti.window >= 64 || !(arrived >> ti.window & 1))) {
                         if (!flag_wait(p.win_ready + ti.window, p.win_ready_target, abort_flag, p.status, kWaitWindowReady, ti.window)) { ok = false; break; }
-                        waited_window = ti.window;
+                        if (ti.window < 64) arrived |= 1ull << ti.window;
                         fenced = true;
                     }
                     if (MODE == FMODE_FWD && ti.phase == 1) {

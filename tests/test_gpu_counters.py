@@ -63,6 +63,24 @@ def test_fused_forward_gemm_equals_the_two_launches_bit_for_bit(rows_per_group, 
     assert done.tolist() == want
 
 
+@pytest.mark.parametrize("blocks,H,I,window", [
+    (41, 1024, 384, 512),         # the down tiles follow six super-groups behind, the last super-group is partial
+    (22, 768, 128, 256),          # fewer super-groups than that: every gate/up tile comes first
+    (49, 1024, 512, 0),           # one long window: gate/up tiles, then down tiles
+])
+def test_fused_forward_gemm_in_every_tile_order(blocks, H, I, window):
+    from mok import _C
+    p = problem([256] * (blocks - 6) + [1536], H, I, seed=73)
+    ref = separate(_C, p)
+    got = outputs(p, fill=3.0)
+    blk = torch.zeros(blocks, dtype=torch.int32, device="cuda")
+    _C.grouped_gemm(4, p["x"], p["Wg"], got[0], group_of_block=p["gob"], G=p["G"], N=I, K=H, B2=p["Wu"], D2=got[1], D3=got[2],
+                    B3=p["Wd"], D4=got[3], N2=H, window_rows=window, blk_done=blk)
+    torch.cuda.synchronize()
+    assert _C.check_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(ref, got))
+
+
 def test_fused_forward_gemm_without_the_down_projection():
     from mok import _C
     p = problem([512, 768], 512, 256, seed=71)
