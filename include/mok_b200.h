@@ -417,6 +417,8 @@ typedef struct {
     /* A launch with win_ready leaves this many SMs (0 = 2) to the kernels that produce the rows it waits for (the
      * reference sets whole SMs aside for communication: num_comm_sms).  The layer uses 2. */
     int reserve_sms;
+    /* mode 2, optional, device [G]: as in mokb_gemm_args, in steps of 128 tokens */
+    const int32_t* group_k_end;
 } mokb_gemm_fp8_args;
 int mokb_grouped_gemm_mxfp8(const mokb_gemm_fp8_args* args, void* stream);
 

@@ -62,6 +62,7 @@ struct FParams {
     const int32_t* num_rows;
     const int32_t* group_of_block;
     const int32_t* group_offsets;
+    const int32_t* group_k_end;      // FMODE_WGRAD, optional: tokens of group g from here on are zero in both operands
     int G, M, N, K;
     int b_rows_per_group;
     int dual;
@@ -140,7 +141,9 @@ struct Sched {
             ti.m_blk = rem - ti.n_blk * m_blocks;
             const int c0 = p.group_offsets[ti.group];
             ti.k_tile0 = c0 / BKB - p.k_tile_origin;
-            ti.k_iters = (p.group_offsets[ti.group + 1] - c0) / BKB;
+            int k_end = p.group_offsets[ti.group + 1];
+            if (p.group_k_end) k_end = min(k_end, max(p.group_k_end[ti.group], c0));
+            ti.k_iters = (k_end - c0 + BKB - 1) / BKB;           // a partial last stage multiplies tokens that are zero
         } else if (MODE == FMODE_FWD) {
             int first_blk = 0, blocks = m_blocks, x;             // the row tiles that x, a tile's number in its phase, counts
             if (lag > 0) {
@@ -657,6 +660,7 @@ extern "C" int mokb_grouped_gemm_mxfp8(const mokb_gemm_fp8_args* g, void* stream
     p.num_rows = g->num_rows;
     p.group_of_block = g->group_of_block;
     p.group_offsets = g->group_offsets;
+    p.group_k_end = g->mode == FMODE_WGRAD ? g->group_k_end : nullptr;
     p.G = g->G; p.M = g->M; p.N = g->N; p.K = g->K;
     p.D = static_cast<__nv_bfloat16*>(g->D);
     p.D2 = static_cast<__nv_bfloat16*>(g->D2);

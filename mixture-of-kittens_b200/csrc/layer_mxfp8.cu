@@ -348,9 +348,11 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
         f.push_values = d_w_row; f.push_value_ptrs_host = a->d_router_weight_ptrs_host;
         MOKB_TRY(mokb_grouped_gemm_mxfp8(&f, stream));
         const int32_t* offs = s.mb_offsets + static_cast<size_t>(m) * (E_l + 1);
+        const int32_t* k_end = s.mb_k_end + static_cast<size_t>(m) * (E_l + 1);
         auto wgrad_fp8 = [&](const void* A, const void* A_sc, int M, const void* B, const void* B_sc, int N, void* D) -> int {
             mokb_gemm_fp8_args w = fp8_base(a->status);
             w.mode = 2; w.rows_static = MB; w.t_first = lo; w.G = E_l; w.M = M; w.N = N; w.group_offsets = offs; w.accumulate = m > 0;
+            w.group_k_end = k_end;       // a segment's padding may fill a whole 128-token stage of zeros
             w.A = A; w.A_sc = A_sc; w.B = B; w.B_sc = B_sc; w.D = D; w.ldd = N;
             return mokb_grouped_gemm_mxfp8(&w, stream);
         };

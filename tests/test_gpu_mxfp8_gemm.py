@@ -147,6 +147,39 @@ def test_mxfp8_gemm_wgrad(cols_per_group, M, N):
         assert_close(f"wgrad {gi}", ref, D[gi], (GEMM_TOL[0] * 8, GEMM_TOL[1]))
 
 
+def test_mxfp8_gemm_wgrad_leaves_out_the_padding_tokens_it_is_told_about():
+    """group_k_end: tokens of a group from there on are zero in both operands.  The kernel stops at the next multiple of
+    128 tokens, so whatever lies beyond that -- E4M3 NaN here -- must not reach the result."""
+    from mok import _C
+    cols_per_group, real, M, N = [512, 768, 0, 256, 256], [257, 640, 0, 1, 256], 256, 384
+    offs, gob, cols = groups(cols_per_group)
+    o = offs.cpu().numpy()
+    k_end = torch.tensor([int(o[i]) + real[i] for i in range(5)], dtype=torch.int32, device="cuda")
+    g = torch.Generator().manual_seed(34)
+    A = torch.randn(M, cols, generator=g).to(torch.bfloat16)
+    B = torch.randn(N, cols, generator=g).to(torch.bfloat16)
+    for i in range(5):
+        A[:, int(o[i]) + real[i]:int(o[i + 1])] = 0
+        B[:, int(o[i]) + real[i]:int(o[i + 1])] = 0
+    Aq, As, Ad = quant(A)
+    Bq, Bs, Bd = quant(B)
+    for i in range(5):
+        s = int(o[i]) + (real[i] + 127) // 128 * 128
+        for q in (Aq, Bq):
+            q.view(torch.uint8)[:, s:int(o[i + 1])] = 0x7F
+    D = torch.full((5, M, N), 5.0, dtype=torch.bfloat16, device="cuda")
+    _C.grouped_gemm_mxfp8(2, Aq, As, Bq, Bs, D, group_offsets=offs, G=5, M=M, N=N, group_k_end=k_end)
+    torch.cuda.synchronize()
+    assert _C.check_status() == 0
+    for i in range(5):
+        s, e = int(o[i]), int(o[i]) + real[i]
+        if real[i] == 0:
+            assert torch.all(D[i] == 0)
+            continue
+        ref = (Ad[:, s:e] @ Bd[:, s:e].T).to(torch.bfloat16)
+        assert_close(f"wgrad {i}", ref, D[i], (GEMM_TOL[0] * 8, GEMM_TOL[1]))
+
+
 @pytest.mark.parametrize("rows_per_group,H,I,window,push", [([512, 256, 0, 768], 512, 384, 512, False),
                                                             ([2048, 512, 3072], 768, 512, 1024, True)])
 def test_mxfp8_fused_forward_equals_the_two_launches_bit_for_bit(rows_per_group, H, I, window, push):
