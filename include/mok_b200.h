@@ -231,7 +231,7 @@ typedef struct {
     void *hidden_fp8_t, *hidden_sc_t;                                         /* [I, MB] */
     void *y_shared, *y_routed;                                                /* [T, H], [MB, H] bf16 */
     /* work */
-    void *x_routed;                                                           /* [MB, H] bf16 */
+    void *x_routed;                                                           /* not used */
     void *x_fp8, *x_sc;                                                       /* [MB, H] */
     void *hidden_fp8, *hidden_sc;                                             /* [MB, I] */
     void* scratch;                                                            /* mokb_layer_scratch_bytes() */
@@ -274,7 +274,7 @@ typedef struct {
     void *d_y_fp8, *d_y_sc;                                                   /* [MB, H] */
     void *d_w_shared_gate, *d_w_routed_gate, *d_w_shared_up, *d_w_routed_up, *d_w_shared_down, *d_w_routed_down;   /* bf16 */
     /* work */
-    void *d_y_routed;                                                         /* [MB, H] bf16 */
+    void *d_y_routed;                                                         /* not used */
     void *d_y_fp8_t, *d_y_sc_t;                                               /* [H, MB] */
     void *d_gate_fp8_t, *d_gate_sc_t, *d_up_fp8_t, *d_up_sc_t;                /* [I, MB] */
     void *partials;                                                           /* [MB, I/128] f32 */
@@ -282,7 +282,7 @@ typedef struct {
      * the context buffers, which it therefore overwrites, ops.py:785-791 of the reference).  Required only when
      * schedule_capacity > macrobatch_size; null otherwise. */
     const void *w_routed_gate, *w_routed_gate_sc, *w_routed_up, *w_routed_up_sc;   /* forward weights, quantised along H */
-    void *x_routed;                                                           /* [MB, H] bf16 */
+    void *x_routed;                                                           /* not used */
     void *x_fp8, *x_sc;                                                       /* [MB, H] */
     void *hidden_fp8, *hidden_sc;                                             /* [MB, I] */
     void* scratch;
@@ -305,13 +305,14 @@ int mokb_struct_sizes_mxfp8(int* out, int n);
  * Weight-gradient GEMM (mode 3): for each group g with rows [off[g], off[g+1]) of
  * A [rows, M] and B [rows, N]: D[g] [M, N] = A_g^T * B_g (zero if the group is empty).
  *   mode 4: mode 1 followed by the down projection of the same rows, D4 [rows, N2] = D3 * B3[g]^T with B3 [G, N2, N],
- *           in ONE persistent launch that walks the rows window by window (window_rows rows each): all gate/up tiles of
- *           a window, then all its down tiles -- the task order of the reference's forward megakernel
- *           (csrc/megakernel/forward.cuh:146-266).  N2 = 0 leaves the down projection out.
+ *           in ONE persistent launch that walks the rows in order, the down tiles a few super-groups of 1024 rows behind the
+ *           gate/up tiles (windows long enough: all gate/up tiles of a window, then all its down tiles -- the task order of
+ *           the reference's forward megakernel, csrc/megakernel/forward.cuh:146-266).  N2 = 0 leaves the down projection out.
  * Counters (modes 0, 1, 2, 4; device int32 arrays that the caller zeroes; the reference's barrier_wait / barrier_arrive,
  * csrc/megakernel/utils.cuh:1-13, with a 2 s limit after which the kernel sets MOKB_ST_FLAG_TIMEOUT and exits):
  *   win_ready[w] -- awaited (>= win_ready_target) before the first A rows of window w (counted from row_begin) are read;
- *                   mokb_dispatch_rows_window adds 1 per block when its rows have landed;
+ *                   mokb_dispatch_rows_window adds 1 per block when its rows have landed; a negative target counts
+ *                   arrivals per 256 rows: a window is ready at -win_ready_target for every 256-row block that it holds;
  *   blk_done[b]  -- mode 4, required, [rows / 256 from row_begin]: the kernel's own count of finished gate/up tiles per
  *                   256-row block, awaited by its down tiles;
  *   win_done[w]  -- mode 4, optional: 8 arrivals per finished down tile of window w; mokb_combine_rows_window waits
@@ -463,6 +464,14 @@ int mokb_dispatch_rows_window(const uint64_t* src_ptrs_host, int ep_size, const 
                               const uint64_t* row_scale_ptrs_host, float* row_scale_out, int blocks,
                               int32_t* done_counter, void* q_out, void* q_sc_out, int64_t index_limit, int32_t* status,
                               void* stream);
+/* The pull that the MXFP8 layer uses: the rows in both MXFP8 forms (q [max_rows, hidden] + sc along columns, qt [hidden, t_rows]
+ * + sct along rows; hidden a multiple of 256), the bf16 rows themselves are not stored.  With a ticket (device int32, zero)
+ * the launch takes the rows in order and raises window_ready[w] by hidden / 32 per 256 rows of window w. */
+int mokb_dispatch_rows_quant(const uint64_t* src_ptrs_host, int ep_size, const int32_t* peer_rank, const int32_t* peer_token_idx,
+                             const int32_t* num_rows, int max_rows, int row_begin, int row_end, int row_divisor, int64_t hidden,
+                             const uint64_t* row_scale_ptrs_host, float* row_scale_out, void* q, void* sc, void* qt, void* sct,
+                             int64_t t_rows, int blocks, int32_t* ticket, int32_t* window_ready, int window_rows,
+                             int64_t index_limit, int32_t* status, void* stream);
 int mokb_combine_rows_window(const void* src, const uint64_t* dst_ptrs_host, int ep_size,
                              const int32_t* peer_rank, const int32_t* peer_token_idx,
                              const int32_t* num_rows, int max_rows, int row_begin, int row_end, int64_t hidden,

@@ -94,6 +94,29 @@ struct RowQuant {
     int col_tiles;          // H / 128
 };
 
+// A launch that feeds a running GEMM: its warps take pieces of the row window from `ticket` (zero at launch) in order, so
+// that the rows arrive in order however many of the blocks are resident at a time, and count what they have finished in
+// window_ready[window].  One launch serves all windows (there used to be one per window: at 256 rows a window the sixteen
+// launches cost four times as much as the copies).
+struct PullOrder {
+    int32_t* ticket;             // null: a fixed share of the rows per warp, nothing counted
+    int32_t* window_ready;
+    int window_rows;             // a multiple of 256
+};
+__device__ __forceinline__ int take_ticket(int32_t* ticket) {
+    int v = 0;
+    if ((threadIdx.x & 31) == 0) v = atomicAdd(ticket, 1);
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+// the whole warp's stores so far are counted as `n` arrivals (a GEMM acquires the counter before it reads the rows)
+__device__ __forceinline__ void count_arrivals(int32_t* counter, int n) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        __threadfence();
+        red_release_gpu_add(counter, n);
+    }
+}
+
 // One warp per schedule row, 16- or 32-byte accesses, four loads in flight per lane.  QUANT (32-byte accesses only):
 // the row is also quantised along its columns from the registers it passes through -- a lane holds 16 consecutive
 // values, two neighbouring lanes one 32-value block (the reference quantises the tile it has just pulled,
@@ -103,7 +126,7 @@ __global__ void __maxnreg__(64) dispatch_kernel(PeerPtrs src, PeerPtrs scale_src
                                 const int32_t* __restrict__ peer_token_idx, const int32_t* __restrict__ num_rows,
                                 int max_rows, int row_begin, int row_end, int R, int row_divisor, int vec_per_row,
                                 Words<W>* __restrict__ dst, float* __restrict__ row_scale_out, int32_t* done_counter, RowQuant rq,
-                                IndexGuard guard) {
+                                IndexGuard guard, PullOrder order) {
     int rows = num_rows ? *num_rows : max_rows;
     rows = rows < 0 ? 0 : (rows > max_rows ? 0 : rows);
     rows = min(rows, row_end);
@@ -113,7 +136,16 @@ __global__ void __maxnreg__(64) dispatch_kernel(PeerPtrs src, PeerPtrs scale_src
     const int nwarps = gridDim.x * warps_per_block;
     // The indices (and the remote scale) of a warp's next row are fetched while it moves the current one: three
     // dependent round trips (indices, scale over NVLink, data over NVLink) would otherwise sit in front of every row.
-    int row = row_begin + warp;
+    // Rows go in pieces of 1 << piece: one row at a fixed stride, or, by ticket, as many as leave every warp a few pieces
+    // (a piece costs its warp a fence: about a microsecond).
+    int piece = 0;
+    if (order.ticket) {
+        const int share = (rows - row_begin) / nwarps;
+        piece = share >= 32 ? 3 : share >= 8 ? 2 : share >= 2 ? 1 : 0;
+    }
+    int cur = order.ticket ? take_ticket(order.ticket) : warp;
+    int nxt = order.ticket ? take_ticket(order.ticket) : warp + nwarps;
+    int row = row_begin + (cur << piece);
     int pr_next = -1, tok_next = 0;
     float w_next = 1.f;
     auto fetch_indices = [&](int r) {
@@ -126,11 +158,23 @@ __global__ void __maxnreg__(64) dispatch_kernel(PeerPtrs src, PeerPtrs scale_src
         }
     };
     fetch_indices(row);
-    for (; row < rows; row += nwarps) {
+    int done = -1;               // the piece whose last row has been stored but not yet counted
+    for (int next_row; row < rows; row = next_row) {
+        if (done >= 0) {
+            count_arrivals(order.window_ready + (done << piece) / order.window_rows, 1 << piece);
+            done = -1;
+        }
         const int pr = pr_next;
         const int tok = tok_next;
         const float w = SCALE ? w_next : 1.f;
-        fetch_indices(row + nwarps);
+        next_row = row + 1;
+        if ((next_row - row_begin) >> piece != cur) {
+            if (order.ticket) done = cur;
+            cur = nxt;
+            nxt = order.ticket ? take_ticket(order.ticket) : nxt + nwarps;
+            next_row = row_begin + (cur << piece);
+        }
+        fetch_indices(next_row);
         Words<W>* out = dst + static_cast<size_t>(row) * vec_per_row;
         if (pr < 0 || pr >= R) {      // padding row (or a rank outside the pointer list: treated as padding, never dereferenced)
             Words<W> zero;
@@ -195,12 +239,187 @@ __global__ void __maxnreg__(64) dispatch_kernel(PeerPtrs src, PeerPtrs scale_src
             }
         }
     }
+    if (done >= 0) count_arrivals(order.window_ready + (done << piece) / order.window_rows, 1 << piece);
     if (done_counter) {      // this block's rows of the window have landed: one arrival for whoever consumes them
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
             red_release_gpu_add(done_counter, 1);
         }
+    }
+}
+
+// Row pull with both MXFP8 forms of the rows -- along columns (q, sc: what the row-tiled GEMMs read) and along tokens
+// (qt, sct: what the weight gradients read) -- from the one read of each value: the bf16 rows are not stored.  (A pull
+// that stored them and a second pass that read them twice for the token-wise form moved 8 bytes per value instead of 4.)
+// A warp works on 32 rows x 32 columns at a time: a half-warp holds 16 rows, a lane two adjacent columns of them, so the
+// token-wise block maximum is local but for one shuffle, and the column-wise maxima of 16 rows over 16 lanes take eight
+// shuffles of packed pairs (half of the values change lanes at each step).  Few warps fit beside a GEMM, so everything that
+// takes a round trip to memory is asked for ahead: the next 32 columns while these are worked on, the next unit's ticket,
+// indices and first columns before this one is counted.  At most 128 registers and no shared memory: one block of 128
+// threads fits beside any of the GEMMs.  The values are those of quantize_kernel, byte for byte.
+struct TokenQuant {
+    uint8_t *q, *sc, *qt, *sct;
+    int64_t t_rows;              // token columns of qt
+};
+constexpr int kQuantRows = 32, kQuantCols = 256;
+
+// 32 rows (lane i knows row i's address) x 32 columns: v[i] = columns col, col + 1 of row i of the half-warp's 16.  The loads
+// are unconditional: a load under a predicate is waited for where it stands (all of them cost a round trip each).
+__device__ __forceinline__ void pull_columns(uint32_t (&v)[16], const uint32_t* row_ptr, int col) {
+    const int base = threadIdx.x & 16;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(row_ptr), base | i));
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(v[i]) : "l"(p + (col >> 1)));
+    }
+}
+
+template <bool SCALE>
+__device__ __forceinline__ void quantize_columns(uint32_t (&v)[16], uint32_t live, float w, int r0, int col, int hidden, const TokenQuant& tq) {
+    const int lane = threadIdx.x & 31, base = lane & 16;
+    if (live != 0xffffffffu) {        // padding rows: whatever was loaded in their place
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = (live >> (base | i)) & 1u ? v[i] : 0u;
+    }
+    if (SCALE) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float f = __shfl_sync(0xffffffffu, w, base | i);
+            v[i] = pack2(bf16_lo(v[i]) * f, bf16_hi(v[i]) * f);
+        }
+    }
+    {      // along tokens: this lane's 16 rows and those of the lane 16 away are one block of each of its two columns
+        uint32_t m = 0u;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) m = absmax2(m, v[i]);
+        m = absmax2(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        float inv_a, inv_b;
+        const uint32_t byte_a = scale_byte(bf16_lo(m), &inv_a);
+        const uint32_t byte_b = scale_byte(bf16_hi(m), &inv_b);
+        uint8_t* dst = tq.qt + col * tq.t_rows + r0 + base;
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            o[i] = e4m3x4(bf16_lo(v[4 * i]) * inv_a, bf16_lo(v[4 * i + 1]) * inv_a, bf16_lo(v[4 * i + 2]) * inv_a, bf16_lo(v[4 * i + 3]) * inv_a);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            o[i] = e4m3x4(bf16_hi(v[4 * i]) * inv_b, bf16_hi(v[4 * i + 1]) * inv_b, bf16_hi(v[4 * i + 2]) * inv_b, bf16_hi(v[4 * i + 3]) * inv_b);
+        *reinterpret_cast<uint4*>(dst + tq.t_rows) = make_uint4(o[0], o[1], o[2], o[3]);
+        // the half-warps write the scale of one of the two columns each
+        tq.sct[scale_offset(col + (base >> 4), r0 >> 5, tq.t_rows >> 7)] = static_cast<uint8_t>(base ? byte_b : byte_a);
+    }
+    // along columns: the 16 lanes of a half-warp hold one block of each of its rows
+    uint32_t p[8];       // p[i]: this lane's maxima of rows i (low half) and i + 8 (high half)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t lo = __byte_perm(v[i], v[i + 8], 0x5410), hi = __byte_perm(v[i], v[i + 8], 0x7632);
+        p[i] = absmax2(lo & 0x7fff7fffu, hi);
+    }
+#pragma unroll
+    for (int half = 4; half >= 1; half >>= 1) {
+        const bool upper = (lane & half) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const uint32_t give = upper ? p[i] : p[i + half], keep = upper ? p[i + half] : p[i];
+            p[i] = absmax2(keep, __shfl_xor_sync(0xffffffffu, give, half));
+        }
+    }
+    p[0] = absmax2(p[0], __shfl_xor_sync(0xffffffffu, p[0], 8));
+    // lane l now has the block maxima of rows l % 8 and l % 8 + 8 of its half-warp; it works out one of the two scales
+    const bool second = (lane & 8) != 0;
+    float inv;
+    const uint32_t byte = scale_byte(second ? bf16_hi(p[0]) : bf16_lo(p[0]), &inv);
+    tq.sc[scale_offset(r0 + base + (lane & 15), col >> 5, hidden >> 7)] = static_cast<uint8_t>(byte);
+    uint8_t* dst = tq.q + static_cast<int64_t>(r0 + base) * hidden + col;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float f = __shfl_sync(0xffffffffu, inv, base | i);
+        uint16_t pair;
+        asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(pair) : "f"(bf16_lo(v[i]) * f), "f"(bf16_hi(v[i]) * f));
+        *reinterpret_cast<uint16_t*>(dst + static_cast<int64_t>(i) * hidden) = pair;
+    }
+}
+
+template <bool SCALE>
+__global__ void __maxnreg__(128) pull_quant_kernel(const __grid_constant__ PeerPtrs src, const __grid_constant__ PeerPtrs scale_src, const int32_t* __restrict__ peer_rank,
+                                                   const int32_t* __restrict__ peer_token_idx, const int32_t* __restrict__ num_rows,
+                                                   int max_rows, int row_begin, int row_end, int R, int row_divisor, int hidden,
+                                                   float* __restrict__ row_scale_out, TokenQuant tq, IndexGuard guard, PullOrder order) {
+    int rows = num_rows ? *num_rows : max_rows;
+    rows = rows < 0 ? 0 : (rows > max_rows ? 0 : rows);
+    rows = min(rows, row_end);
+    const int lane = threadIdx.x & 31;
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    // a unit: 32 rows x 256, 512 or 1024 columns, as many as leave every warp a few units (counting one costs a fence)
+    const int groups = rows > row_begin ? (rows - row_begin + kQuantRows - 1) / kQuantRows : 0;
+    const int share = static_cast<int>(static_cast<int64_t>(groups) * (hidden / kQuantCols) / nwarps);
+    const int unit_cols = kQuantCols << (share >= 32 ? 2 : share >= 16 ? 1 : 0);
+    const int col_units = (hidden + unit_cols - 1) / unit_cols;
+    const int units = groups * col_units;
+    // row r0 + lane of a unit: its rank and route, then (a second round trip) its address and scale
+    int pr = -1, tok = 0;
+    auto look_up = [&](int unit) {
+        const int row = row_begin + unit / col_units * kQuantRows + lane;
+        pr = -1;
+        if (unit < units && row < rows) {
+            pr = peer_rank[row];
+            tok = peer_token_idx[row];
+        }
+    };
+    struct Rows {
+        const uint32_t* ptr;         // of this lane's row; of a scheduled row of the unit if it is padding
+        uint32_t live;               // which of the 32 rows are scheduled (none: nothing is loaded)
+        float w;
+    };
+    auto resolve = [&](int unit) {
+        Rows out;
+        out.ptr = nullptr;
+        out.w = 0.f;
+        if (pr >= 0 && pr < R && index_ok(guard, tok, kBadIndexPull, row_begin + unit / col_units * kQuantRows + lane)) {
+            out.ptr = static_cast<const uint32_t*>(src.p[pr]) + static_cast<size_t>(tok / row_divisor) * (hidden / 2);
+            if (SCALE) out.w = static_cast<const float*>(scale_src.p[pr])[tok];
+        }
+        out.live = __ballot_sync(0xffffffffu, out.ptr != nullptr);
+        const unsigned long long any = __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(out.ptr), __ffs(out.live | 0x80000000u) - 1);
+        if (out.ptr == nullptr) out.ptr = reinterpret_cast<const uint32_t*>(any);
+        return out;
+    };
+    auto next_unit = [&](int u) { return order.ticket ? take_ticket(order.ticket) : u + nwarps; };
+    int unit = order.ticket ? take_ticket(order.ticket) : static_cast<int>(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+    if (unit >= units) return;
+    look_up(unit);
+    Rows cur = resolve(unit);
+    uint32_t va[16], vb[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) va[i] = vb[i] = 0u;
+    const int lane_col = 2 * (lane & 15);
+    if (cur.live) pull_columns(va, cur.ptr, unit % col_units * unit_cols + lane_col);
+    while (unit < units) {
+        const int g = unit / col_units;
+        const int c0 = (unit - g * col_units) * unit_cols, c1 = min(c0 + unit_cols, hidden);
+        const int r0 = row_begin + g * kQuantRows;
+        if (SCALE && c0 == 0 && row_scale_out && r0 + lane < rows) row_scale_out[r0 + lane] = cur.w;
+        int next = 0;
+        Rows nxt = {nullptr, 0u, 0.f};
+#pragma unroll 1
+        for (int c = c0; c < c1; c += 64) {            // (at least four trips: the columns are a multiple of 256)
+            if (cur.live) pull_columns(vb, cur.ptr, c + 32 + lane_col);
+            if (c == c0) next = next_unit(unit);
+            if (c == c0 + 64) look_up(next);
+            if (c + 64 == c1) nxt = resolve(next);
+            quantize_columns<SCALE>(va, cur.live, cur.w, r0, c + lane_col, hidden, tq);
+            if (c + 64 < c1) {
+                if (cur.live) pull_columns(va, cur.ptr, c + 64 + lane_col);
+            } else if (nxt.live) {
+                pull_columns(va, nxt.ptr, next % col_units * unit_cols + lane_col);
+            }
+            quantize_columns<SCALE>(vb, cur.live, cur.w, r0, c + 32 + lane_col, hidden, tq);
+        }
+        if (order.ticket) count_arrivals(order.window_ready + g * kQuantRows / order.window_rows, (c1 - c0) / kQuantCols);
+        unit = next;
+        cur = nxt;
     }
 }
 
@@ -325,7 +544,7 @@ int dispatch_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32_t
                        const int32_t* peer_token_idx, const int32_t* num_rows, int max_rows, int row_begin, int row_end,
                        int row_divisor, int64_t hidden, void* dst, const uint64_t* row_scale_ptrs_host,
                        float* row_scale_out, int blocks, cudaStream_t s, int32_t* done_counter, void* q_out, void* q_sc_out,
-                       int64_t index_limit, int32_t* status) {
+                       int64_t index_limit, int32_t* status, int32_t* ticket, int window_rows) {
     TraceScope trace(s, row_scale_ptrs_host ? "dispatch_scaled" : "dispatch", row_begin);
     MOKB_REQUIRE((q_out == nullptr) == (q_sc_out == nullptr), "dispatch_rows: the quantised rows and their scales go together");
     MOKB_REQUIRE(ep_size >= 1 && ep_size <= MOKB_MAX_EP, "dispatch_rows: bad ep_size");
@@ -356,10 +575,10 @@ int dispatch_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32_t
     }
 #define MOKB_DISPATCH(SC, WW, QQ)                                                                                              \
     do {                                                                                                                       \
-        share_sms_with_gemm(dispatch_kernel<SC, WW, QQ>);                                                                      \
+        share_sms_with_gemm<dispatch_kernel<SC, WW, QQ>>();                                                                    \
         dispatch_kernel<SC, WW, QQ><<<blocks, threads, 0, s>>>(src, scale, peer_rank, peer_token_idx, num_rows, max_rows,      \
             row_begin, row_end, ep_size, row_divisor, vec, static_cast<Words<WW>*>(dst), SC ? row_scale_out : nullptr,         \
-            done_counter, rq, guard);                                                                                          \
+            ticket ? nullptr : done_counter, rq, guard, PullOrder{ticket, done_counter, window_rows});                                                                                          \
     } while (0)
     if (row_scale_ptrs_host) {
         if (q_out) MOKB_DISPATCH(true, 8, true);
@@ -371,6 +590,45 @@ int dispatch_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32_t
         else MOKB_DISPATCH(false, 4, false);
     }
 #undef MOKB_DISPATCH
+    MOKB_CUDA(cudaGetLastError());
+    note_launch();
+    return MOKB_OK;
+}
+
+// Arrivals that pull_quant_rows_impl counts per 256 rows (dispatch_rows_impl by ticket: 256).
+int pull_quant_arrivals(int64_t hidden) { return static_cast<int>(256 / kQuantRows * (hidden / kQuantCols)); }
+
+// Rows [row_begin, row_end) from their home ranks into both MXFP8 forms (q / sc, qt / sct addressed by schedule row;
+// qt has t_rows token columns).  ticket / window_ready / window_rows: see PullOrder.
+int pull_quant_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32_t* peer_rank, const int32_t* peer_token_idx,
+                         const int32_t* num_rows, int max_rows, int row_begin, int row_end, int row_divisor, int64_t hidden,
+                         const uint64_t* row_scale_ptrs_host, float* row_scale_out, void* q, void* sc, void* qt, void* sct, int64_t t_rows,
+                         int blocks, cudaStream_t s, int32_t* ticket, int32_t* window_ready, int window_rows, int64_t index_limit,
+                         int32_t* status) {
+    TraceScope trace(s, row_scale_ptrs_host ? "dispatch_quant_scaled" : "dispatch_quant", row_begin);
+    MOKB_REQUIRE(ep_size >= 1 && ep_size <= MOKB_MAX_EP && peer_rank && peer_token_idx && q && sc && qt && sct, "pull_quant_rows: null pointer");
+    MOKB_REQUIRE(hidden > 0 && hidden % kQuantCols == 0 && row_divisor >= 1 && row_begin >= 0 && row_begin <= row_end && row_begin % 128 == 0 && t_rows % 128 == 0,
+                 "pull_quant_rows: bad sizes");
+    MOKB_REQUIRE((reinterpret_cast<uintptr_t>(q) & 1) == 0 && (reinterpret_cast<uintptr_t>(qt) & 31) == 0, "pull_quant_rows: outputs not aligned");
+    MOKB_REQUIRE(ticket == nullptr || (window_ready && window_rows > 0 && window_rows % 256 == 0), "pull_quant_rows: a ticket needs windows");
+    MOKB_REQUIRE(index_limit >= 0 && index_limit <= INT32_MAX && (index_limit == 0 || status != nullptr), "pull_quant_rows: bad index limit");
+    PeerPtrs src, scale;
+    MOKB_TRY(fill_peers(&src, src_ptrs_host, ep_size, "src_ptrs"));
+    for (int r = 0; r < kPeerMax; ++r) scale.p[r] = nullptr;
+    for (int r = 0; r < ep_size && row_scale_ptrs_host; ++r) {
+        MOKB_REQUIRE(row_scale_ptrs_host[r] != 0, "pull_quant_rows: null scale pointer for rank %d", r);
+        scale.p[r] = reinterpret_cast<void*>(static_cast<uintptr_t>(row_scale_ptrs_host[r]));
+    }
+    if (max_rows == 0 || row_begin >= max_rows) return MOKB_OK;
+    if (blocks <= 0) blocks = comm_default_blocks();
+    const TokenQuant tq{static_cast<uint8_t*>(q), static_cast<uint8_t*>(sc), static_cast<uint8_t*>(qt), static_cast<uint8_t*>(sct), t_rows};
+    const IndexGuard guard{static_cast<int>(index_limit), status};
+    const PullOrder order{ticket, window_ready, window_rows};
+    auto kernel = row_scale_ptrs_host ? pull_quant_kernel<true> : pull_quant_kernel<false>;
+    if (row_scale_ptrs_host) share_sms_with_gemm<pull_quant_kernel<true>>();
+    else share_sms_with_gemm<pull_quant_kernel<false>>();
+    kernel<<<blocks, 128, 0, s>>>(src, scale, peer_rank, peer_token_idx, num_rows, max_rows, row_begin, row_end, ep_size, row_divisor,
+                                  static_cast<int>(hidden), row_scale_out, tq, guard, order);
     MOKB_CUDA(cudaGetLastError());
     note_launch();
     return MOKB_OK;
@@ -400,8 +658,8 @@ int combine_rows_impl(const void* src, const uint64_t* dst_ptrs_host, int ep_siz
         }
     if (max_rows == 0 || row_begin >= max_rows) return MOKB_OK;
     if (blocks <= 0) blocks = comm_default_blocks();
-    share_sms_with_gemm(combine_kernel<8>);
-    share_sms_with_gemm(combine_kernel<4>);
+    share_sms_with_gemm<combine_kernel<8>>();
+    share_sms_with_gemm<combine_kernel<4>>();
     if (rows_aligned32(src, dst, ep_size, hidden))
         combine_kernel<8><<<blocks, 128, 0, s>>>(static_cast<const Words<8>*>(src), dst, val, peer_rank, peer_token_idx, num_rows, max_rows,
                                                  row_begin, row_end, ep_size, static_cast<int>(hidden / 16), row_values, wait_counter,
@@ -436,6 +694,16 @@ extern "C" int mokb_dispatch_rows_window(const uint64_t* src_ptrs_host, int ep_s
     return dispatch_rows_impl(src_ptrs_host, ep_size, peer_rank, peer_token_idx, num_rows, max_rows, row_begin, row_end, row_divisor,
                               hidden, dst, row_scale_ptrs_host, row_scale_out, blocks, static_cast<cudaStream_t>(stream), done_counter,
                               q_out, q_sc_out, index_limit, status);
+}
+
+extern "C" int mokb_dispatch_rows_quant(const uint64_t* src_ptrs_host, int ep_size, const int32_t* peer_rank, const int32_t* peer_token_idx,
+                                        const int32_t* num_rows, int max_rows, int row_begin, int row_end, int row_divisor, int64_t hidden,
+                                        const uint64_t* row_scale_ptrs_host, float* row_scale_out, void* q, void* sc, void* qt, void* sct,
+                                        int64_t t_rows, int blocks, int32_t* ticket, int32_t* window_ready, int window_rows,
+                                        int64_t index_limit, int32_t* status, void* stream) {
+    return pull_quant_rows_impl(src_ptrs_host, ep_size, peer_rank, peer_token_idx, num_rows, max_rows, row_begin, row_end, row_divisor, hidden,
+                                row_scale_ptrs_host, row_scale_out, q, sc, qt, sct, t_rows, blocks, static_cast<cudaStream_t>(stream), ticket,
+                                window_ready, window_rows, index_limit, status);
 }
 
 extern "C" int mokb_combine_rows(const void* src, const uint64_t* dst_ptrs_host, int ep_size,

@@ -36,9 +36,9 @@ int sm_count();
 // Kernels that run on the side streams beside a GEMM ask for the same shared-memory / L1 split as the GEMM (all
 // shared memory).  An SM changes its split only when it is empty: blocks of a kernel with the default split that sit
 // on every SM -- above all blocks that WAIT for the GEMM -- would keep its 197 KB CTAs from ever being placed.
-template <class Kernel>
-inline void share_sms_with_gemm(Kernel kernel) {
-    static bool done = false;       // one flag per kernel type
+template <auto kernel>             // the kernel itself: kernels of one signature share a type
+inline void share_sms_with_gemm() {
+    static bool done = false;
     if (!done) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, static_cast<int>(cudaSharedmemCarveoutMaxShared));
         done = true;
@@ -73,7 +73,14 @@ int dispatch_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32_t
                        const int32_t* peer_token_idx, const int32_t* num_rows, int max_rows, int row_begin, int row_end,
                        int row_divisor, int64_t hidden, void* dst, const uint64_t* row_scale_ptrs_host,
                        float* row_scale_out, int blocks, cudaStream_t s, int32_t* done_counter = nullptr,
-                       void* q_out = nullptr, void* q_sc_out = nullptr, int64_t index_limit = 0, int32_t* status = nullptr);
+                       void* q_out = nullptr, void* q_sc_out = nullptr, int64_t index_limit = 0, int32_t* status = nullptr,
+                       int32_t* ticket = nullptr, int window_rows = 0);
+int pull_quant_arrivals(int64_t hidden);
+int pull_quant_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32_t* peer_rank, const int32_t* peer_token_idx,
+                         const int32_t* num_rows, int max_rows, int row_begin, int row_end, int row_divisor, int64_t hidden,
+                         const uint64_t* row_scale_ptrs_host, float* row_scale_out, void* q, void* sc, void* qt, void* sct, int64_t t_rows,
+                         int blocks, cudaStream_t s, int32_t* ticket, int32_t* window_ready, int window_rows, int64_t index_limit,
+                         int32_t* status);
 int combine_rows_impl(const void* src, const uint64_t* dst_ptrs_host, int ep_size, const int32_t* peer_rank,
                       const int32_t* peer_token_idx, const int32_t* num_rows, int max_rows, int row_begin, int row_end,
                       int64_t hidden, const float* row_values, const uint64_t* value_ptrs_host, int blocks, cudaStream_t s,

@@ -131,6 +131,11 @@ struct Sched {
             }
         }
     }
+    // arrivals that make window w complete: a fixed number, or (negative) so many per 256 rows that the window holds
+    __device__ int arrivals(const FParams& p, int w) const {
+        if (p.win_ready_target >= 0) return p.win_ready_target;
+        return -p.win_ready_target * (min(win_blocks, m_blocks - w * win_blocks) * 1);
+    }
     __device__ Tile get(const FParams& p, int t) const {
         Tile ti;
         if (MODE == FMODE_WGRAD) {
@@ -300,7 +305,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
                     // rows that another kernel (or, for a down tile, other CTAs of this one) is still producing
                     bool fenced = false;
                     if (p.win_ready && ti.phase == 0 && (ti.window >= 64 || !(arrived >> ti.window & 1))) {
-                        if (!flag_wait(p.win_ready + ti.window, p.win_ready_target, abort_flag, p.status, kWaitWindowReady, ti.window)) { ok = false; break; }
+                        if (!flag_wait(p.win_ready + ti.window, sched.arrivals(p, ti.window), abort_flag, p.status, kWaitWindowReady, ti.window)) { ok = false; break; }
                         if (ti.window < 64) arrived |= 1ull << ti.window;
                         fenced = true;
                     }
@@ -688,7 +693,7 @@ extern "C" int mokb_grouped_gemm_mxfp8(const mokb_gemm_fp8_args* g, void* stream
     }
     if (g->mode != FMODE_WGRAD) {
         MOKB_REQUIRE(g->window_rows >= 0 && g->window_rows % 256 == 0, "grouped_gemm_mxfp8: window_rows must be a multiple of 256");
-        MOKB_REQUIRE(g->win_ready == nullptr || (g->window_rows > 0 && g->win_ready_target > 0), "grouped_gemm_mxfp8: win_ready needs window_rows and a target");
+        MOKB_REQUIRE(g->win_ready == nullptr || (g->window_rows > 0 && g->win_ready_target != 0), "grouped_gemm_mxfp8: win_ready needs window_rows and a target");
         p.window_rows = g->window_rows;
         p.win_ready = g->win_ready;
         p.win_ready_target = g->win_ready_target;

@@ -4,11 +4,11 @@
 // Nothing here synchronises the host: the number of routed rows is read on the device by every kernel
 // (forward.cuh:20 does the same).
 //
-//   forward   side stream: dispatch(w0) dispatch(w1) ...                      each raises win_ready[w] when its rows have landed
+//   forward   side stream: dispatch, in row order                             raises win_ready[w] as the rows of window w land
 //             caller     : prologue | shared gate/up, shared down | ONE routed launch: for every window w
 //                          { wait win_ready[w]; gate/up + SwiGLU tiles; down tiles, each after the gate/up tiles of its
 //                            256 rows (blk_done); the down epilogue stores every row into its home rank's combine buffer }
-//   backward  side stream: scaled dispatch of d_y in four windows, raising win_ready[w]
+//   backward  side stream: scaled dispatch of d_y, likewise
 //             caller     : prologue | shared backward (6 launches) | d_hidden = d_y * W_down (one launch, window by window)
 //                          | SwiGLU backward | d_x = d_gate * W_gate + d_up * W_up, whose epilogue stores every row and its
 //                            router-weight gradient into the home rank's buffers | three weight gradients
@@ -42,18 +42,12 @@ int get_async(Async** out) {
     MOKB_REQUIRE(dev >= 0 && dev < 64, "layer: device index %d out of range", dev);
     Async& a = g_async[dev];
     if (!a.ready) {
-        // s1 carries the pulls a waiting GEMM depends on, s2 work that is only needed later (the token-wise MXFP8 copies):
-        // where both have blocks ready for the same free slot of an SM, the pull goes first
+        // s1 carries the pulls a waiting GEMM depends on: where both have blocks ready for the same free slot of an SM, the pull goes first
         int prio_low = 0, prio_high = 0;
         MOKB_CUDA(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
         MOKB_CUDA(cudaStreamCreateWithPriority(&a.s1, cudaStreamNonBlocking, prio_high));
-        MOKB_CUDA(cudaStreamCreateWithPriority(&a.s2, cudaStreamNonBlocking, prio_low));
         cudaEvent_t* single[3] = {&a.fork, &a.join1, &a.join2};
         for (auto e : single) MOKB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-        for (int c = 0; c < kMaxChunks; ++c) {
-            MOKB_CUDA(cudaEventCreateWithFlags(&a.ev_in[c], cudaEventDisableTiming));
-            MOKB_CUDA(cudaEventCreateWithFlags(&a.ev_out[c], cudaEventDisableTiming));
-        }
         a.ready = true;
     }
     *out = &a;
@@ -94,20 +88,18 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_bf16(const mokb_fwd_bf16_arg
     Async* as = nullptr;
     if (overlap) MOKB_TRY(get_async(&as));
     cudaStream_t s_in = overlap ? as->s1 : stream;
-    const int comm_blocks = overlap ? a->num_comm_sms * kCommBlocksPerSm : 0;
+    const int comm_blocks = overlap ? comm_block_count(a->num_comm_sms) : 0;
     // recompute only rebuilds macrobatch 0 (the saved context); the forward walks all of them, last first
     const int n_macro = with_down ? macrobatches(C, MB) : 1;
 
     MOKB_TRY(run_prologue(a->tokens_per_expert, a->num_tokens, a->peer_rank, E_l, C, MB, T, s, a->status, stream));
     const void* x_local = reinterpret_cast<const void*>(static_cast<uintptr_t>(a->x_ptrs_host[a->ep_rank]));
-    bool shared_done = false;
 
     for (int mi = 0; mi < n_macro; ++mi) {
         const int m = n_macro - 1 - mi;
         const int lo = m * MB, hi = (lo + MB < C) ? lo + MB : C;
         // only macrobatch 0 (the one that is always populated) is cut into overlap windows
         const int chunk = m == 0 ? chunk_rows_for(MB, a->minibatch_size) : MB;
-        const int nchunks = (hi - lo + chunk - 1) / chunk;
         // windows of macrobatch 0 are tied to the GEMM launch by counters: the GEMM is ONE persistent launch that
         // starts window w when the dispatch blocks of w have arrived
         const bool flags = overlap && m == 0;
@@ -121,17 +113,14 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_bf16(const mokb_fwd_bf16_arg
             MOKB_CUDA(cudaEventRecord(as->fork, stream));
             MOKB_CUDA(cudaStreamWaitEvent(s_in, as->fork, 0));
         }
-        // dispatch: pull every scheduled row from its home rank, window by window
-        for (int c = 0; c < nchunks; ++c) {
-            const int r0 = lo + c * chunk, r1 = r0 + chunk < hi ? r0 + chunk : hi;
-            MOKB_TRY(dispatch_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, r0, r1, a->topk, H,
-                                        x_routed, nullptr, nullptr, comm_blocks, s_in, flags ? s.win_ready + c : nullptr, nullptr, nullptr, routes, a->status));
-        }
+        // dispatch: pull every scheduled row from its home rank, in row order
+        MOKB_TRY(dispatch_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
+                                    x_routed, nullptr, nullptr, comm_blocks, s_in, flags ? s.win_ready : nullptr, nullptr, nullptr, routes, a->status,
+                                    flags ? s.ticket : nullptr, chunk));
         if (overlap) MOKB_CUDA(cudaEventRecord(as->join1, s_in));
 
-        if (!shared_done) {
-            // shared expert: gate/up + SwiGLU in one pass, then down (independent of the dispatch)
-            shared_done = true;
+        if (m == 0) {
+            // shared expert: gate/up + SwiGLU in one pass, then down, under macrobatch 0's dispatch
             mokb_gemm_args g = gemm_base(a->status);
             g.mode = 1; g.rows_static = T; g.N = I; g.K = H;
             g.A = x_local; g.lda = H; g.B = a->w_shared_gate; g.B2 = a->w_shared_up; g.ldb = H;
@@ -156,7 +145,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_bf16(const mokb_fwd_bf16_arg
         g.has_swiglu_limit = a->has_swiglu_limit; g.swiglu_limit = a->swiglu_limit;
         g.window_rows = chunk;
         g.blk_done = s.blk_done + lo / 256;
-        if (flags) { g.win_ready = s.win_ready; g.win_ready_target = comm_blocks; }
+        if (flags) { g.win_ready = s.win_ready; g.win_ready_target = -256; }
         if (with_down) {
             // combine: the epilogue of every down tile stores its rows straight into slot t*K+k of their home ranks'
             // combine buffers (y_routed, when the caller wants it, gets a copy)
@@ -190,7 +179,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
     Async* as = nullptr;
     if (overlap) MOKB_TRY(get_async(&as));
     cudaStream_t s_in = overlap ? as->s1 : stream;
-    const int comm_blocks = overlap ? a->num_comm_sms * kCommBlocksPerSm : 0;
+    const int comm_blocks = overlap ? comm_block_count(a->num_comm_sms) : 0;
     const int lim = a->has_swiglu_limit;
     const float limv = a->swiglu_limit;
     const int n_macro = macrobatches(C, MB);
@@ -232,18 +221,14 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
             MOKB_TRY(dispatch_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
                                         x_routed, nullptr, nullptr, comm_blocks, s_in, nullptr, nullptr, nullptr, routes, a->status));
         if (overlap) MOKB_CUDA(cudaEventRecord(as->join1, s_in));     // the replayed x is in place
-        // reverse combine: pull d_y rows, scaled by the route's router weight, in a few windows; in macrobatch 0 the
-        // first routed GEMM is one launch that starts each window when the window's dispatch blocks have arrived
+        // reverse combine: pull d_y rows, scaled by the route's router weight; in macrobatch 0 the first routed GEMM is one
+        // launch that starts each window when the window's rows have arrived
         const bool flags = overlap && m == 0;
-        const int bchunk = bwd_chunk_rows(hi - lo, m == 0);
-        const int nb = (hi - lo + bchunk - 1) / bchunk;
-        for (int c = 0; c < nb; ++c) {
-            const int r0 = lo + c * bchunk, r1 = r0 + bchunk < hi ? r0 + bchunk : hi;
-            MOKB_TRY(dispatch_rows_impl(a->d_y_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, r0, r1, a->topk, H,
-                                        d_y_r, a->router_weight_ptrs_host, w_row, comm_blocks, s_in, flags ? s.win_ready + c : nullptr, nullptr, nullptr,
-                                        routes, a->status));
-        }
-        if (overlap) MOKB_CUDA(cudaEventRecord(as->ev_in[0], s_in));
+        const int chunk = chunk_rows_for(MB, a->minibatch_size);
+        MOKB_TRY(dispatch_rows_impl(a->d_y_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
+                                    d_y_r, a->router_weight_ptrs_host, w_row, comm_blocks, s_in, flags ? s.win_ready : nullptr, nullptr, nullptr,
+                                    routes, a->status, flags ? s.ticket : nullptr, chunk));
+        if (overlap) MOKB_CUDA(cudaEventRecord(as->join2, s_in));
 
         if (m == 0) {
             // ---- shared expert (overlaps the dispatch above)
@@ -276,15 +261,15 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
             MOKB_TRY(mokb_grouped_gemm_bf16(&g, stream));
         }
         // d_hidden = d_y * W_down, window by window behind the pull
-        if (overlap && !flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->ev_in[0], 0));
+        if (overlap && !flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->join2, 0));
         g = gemm_base(a->status);
         g.mode = 2; g.rows_static = hi; g.row_begin = lo; g.row_end = hi;
         g.num_rows = s.n_rows; g.group_of_block = s.group_of_block; g.G = E_l; g.N = I; g.K = H;
         g.A = d_y_r; g.lda = H; g.B = a->w_routed_down; g.ldb = I; g.D = d_hidden_r; g.ldd = I;
-        if (flags) { g.window_rows = bchunk; g.win_ready = s.win_ready; g.win_ready_target = comm_blocks; }
+        if (flags) { g.window_rows = chunk; g.win_ready = s.win_ready; g.win_ready_target = -256; }
         MOKB_TRY(mokb_grouped_gemm_bf16(&g, stream));
         // (the pulls have all arrived once that GEMM is through its last window; the event makes it formal)
-        if (flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->ev_in[0], 0));
+        if (flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->join2, 0));
         MOKB_TRY(mokb_swiglu_bwd(a->gate_routed, a->up_routed, a->d_hidden_routed, a->d_gate_routed, a->d_up_routed, s.w_row, s.d_w_row,
                                  s.mb_rows + m, MB, I, lim, limv, stream));
         // d_x = d_gate * W_gate + d_up * W_up; the epilogue stores every row straight into slot t*K+k of its home rank's

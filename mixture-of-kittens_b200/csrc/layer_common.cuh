@@ -25,8 +25,8 @@ struct Scratch {
     float* w_row;              // [MB] router weight of each routed row of the current macrobatch (backward)
     float* d_w_row;            // [MB] router-weight gradient of each routed row (backward)
     // counters between kernels that run at the same time (zeroed by the prologue of every call)
-    int32_t* win_ready;        // [kMaxChunks] blocks of the dispatch launch of window w that have finished
-    int32_t* win_done;         // [kMaxChunks] epilogue warps that have stored a down tile of window w
+    int32_t* win_ready;        // [kMaxChunks] arrivals of the rows of window w (comm.cu: PullOrder)
+    int32_t* ticket;           // [1] next piece of rows of the pull that raises them
     int32_t* blk_done;         // [capacity / 256] epilogue warps that have stored a gate/up tile of a 256-row block
 };
 
@@ -34,15 +34,26 @@ inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 inline int macrobatches(int capacity, int MB) { return (capacity + MB - 1) / MB; }
 
-constexpr int kMaxChunks = 32;     // windows per macrobatch (side-stream events, counters)
-// `num_comm_sms` SMs' worth of communication threads: 2048 per SM, in blocks of 128 (see comm.cu)
+constexpr int kMaxChunks = 32;     // windows per macrobatch (counters)
+// `num_comm_sms` SMs' worth of communication threads: 2048 per SM, in blocks of 128 (see comm.cu), but at most two blocks
+// per SM: that many fit beside a CTA of any of the GEMMs (registers per SM quarter), so that the GEMMs, which start while
+// the pull is running, find room on every SM.
 constexpr int kCommBlocksPerSm = 16;
+inline int comm_block_count(int num_comm_sms) {
+    const int wanted = num_comm_sms * kCommBlocksPerSm, fit = 2 * sm_count();
+    return wanted < fit ? wanted : fit;
+}
+// The quantising pull takes 128 registers per thread (32 values stay in registers through both passes): one block per SM.
+inline int quant_comm_block_count(int num_comm_sms) {
+    const int wanted = num_comm_sms * kCommBlocksPerSm;
+    return wanted < sm_count() ? wanted : sm_count();
+}
 
 inline size_t scratch_bytes(int capacity, int E_l, int MB) {
     const size_t nm = macrobatches(capacity, MB);
     return align256((E_l + 1) * 4) + 512 + align256(nm * 4) + 2 * align256(nm * (E_l + 1) * 4) +
            align256(static_cast<size_t>(capacity / 128) * 4) + 2 * align256(static_cast<size_t>(MB) * 4) +
-           2 * align256(kMaxChunks * 4) + align256(static_cast<size_t>(capacity / 256) * 4);
+           align256(kMaxChunks * 4) + 256 + align256(static_cast<size_t>(capacity / 256) * 4);
 }
 
 inline Scratch carve(void* base, int capacity, int E_l, int MB) {
@@ -59,7 +70,7 @@ inline Scratch carve(void* base, int capacity, int E_l, int MB) {
     s.w_row = reinterpret_cast<float*>(p); p += align256(static_cast<size_t>(MB) * 4);
     s.d_w_row = reinterpret_cast<float*>(p); p += align256(static_cast<size_t>(MB) * 4);
     s.win_ready = reinterpret_cast<int32_t*>(p); p += align256(kMaxChunks * 4);
-    s.win_done = reinterpret_cast<int32_t*>(p); p += align256(kMaxChunks * 4);
+    s.ticket = reinterpret_cast<int32_t*>(p); p += 256;
     s.blk_done = reinterpret_cast<int32_t*>(p);
     return s;
 }
@@ -143,7 +154,8 @@ __global__ void prologue_kernel(const int32_t* __restrict__ tokens_per_expert, c
         }
         s.group_of_block[b] = g;
     }
-    for (int i = threadIdx.x; i < kMaxChunks; i += blockDim.x) s.win_ready[i] = s.win_done[i] = 0;
+    for (int i = threadIdx.x; i < kMaxChunks; i += blockDim.x) s.win_ready[i] = 0;
+    if (threadIdx.x == 0) *s.ticket = 0;
     for (int i = threadIdx.x; i < capacity / 256; i += blockDim.x) s.blk_done[i] = 0;
 }
 
@@ -187,10 +199,8 @@ int check_common(const A* a, const char* who) {
 
 struct Async {
     bool ready = false;
-    cudaStream_t s1 = nullptr, s2 = nullptr;
+    cudaStream_t s1 = nullptr;
     cudaEvent_t fork = nullptr, join1 = nullptr, join2 = nullptr;
-    cudaEvent_t ev_in[kMaxChunks] = {nullptr};    // dispatch of window c finished
-    cudaEvent_t ev_out[kMaxChunks] = {nullptr};   // rows of window c are ready to be combined
 };
 
 int get_async(Async** out);      // layer.cu
@@ -203,14 +213,6 @@ inline int chunk_rows_for(int MB, int minibatch) {
     int rows = minibatch;
     if ((MB + rows - 1) / rows > kMaxChunks) rows = static_cast<int>(align256((MB + kMaxChunks - 1) / kMaxChunks));
     return rows;
-}
-
-// The backward pulls d_y in a few large windows, so that the first routed GEMM can start on the rows that have
-// arrived while the rest is still in flight (macrobatch 0 only; later macrobatches are replays of small remainders).
-constexpr int kBwdWindows = 4;
-inline int bwd_chunk_rows(int rows, bool windowed) {
-    if (!windowed || rows <= 0) return rows > 0 ? rows : 256;
-    return static_cast<int>(align256((rows + kBwdWindows - 1) / kBwdWindows));
 }
 
 // Address such that element [row][0] of a [.., ld] buffer holding macrobatch rows from `first_row` on is

@@ -53,16 +53,15 @@ inline void* rebase_scales_t(const void* sc, int first) {
 
 // The routed forward tensors of one macrobatch, addressed by schedule row.
 struct FwdView {
-    void *x_routed, *x_fp8, *x_sc, *x_fp8_t, *x_sc_t;
+    void *x_fp8, *x_sc, *x_fp8_t, *x_sc_t;
     void *gate_fp8, *gate_sc, *up_fp8, *up_sc;
     void *hidden_fp8, *hidden_sc, *hidden_fp8_t, *hidden_sc_t;
 };
 
-FwdView fwd_view(int lo, int H, int I, void* x_routed, void* x_fp8, void* x_sc, void* x_fp8_t, void* x_sc_t,
+FwdView fwd_view(int lo, int H, int I, void* x_fp8, void* x_sc, void* x_fp8_t, void* x_sc_t,
                  void* gate_fp8, void* gate_sc, void* up_fp8, void* up_sc, void* hidden_fp8, void* hidden_sc,
                  void* hidden_fp8_t, void* hidden_sc_t) {
     FwdView v;
-    v.x_routed = rebase(x_routed, lo, 2ull * H);
     v.x_fp8 = rebase(x_fp8, lo, 1ull * H);
     v.x_sc = rebase_scales(x_sc, lo, H);
     v.x_fp8_t = rebase_t(x_fp8_t, lo);
@@ -106,7 +105,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_mxfp8(const mokb_fwd_mxfp8_a
                  a->w_routed_up_sc, "fwd_mxfp8: null input");
     MOKB_REQUIRE(a->x_fp8_t && a->x_sc_t && a->gate_shared && a->up_shared && a->hidden_shared && a->gate_fp8 && a->gate_sc &&
                  a->up_fp8 && a->up_sc && a->hidden_fp8_t && a->hidden_sc_t, "fwd_mxfp8: null output");
-    MOKB_REQUIRE(a->x_routed && a->x_fp8 && a->x_sc && a->hidden_fp8 && a->hidden_sc, "fwd_mxfp8: null work buffer");
+    MOKB_REQUIRE(a->x_fp8 && a->x_sc && a->hidden_fp8 && a->hidden_sc, "fwd_mxfp8: null work buffer");
     const bool with_down = !a->skip_down_combine;
     if (with_down)
         MOKB_REQUIRE(a->combine_ptrs_host && a->w_shared_down && a->w_routed_down && a->w_routed_down_sc && a->y_shared,
@@ -119,15 +118,13 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_mxfp8(const mokb_fwd_mxfp8_a
     Async* as = nullptr;
     if (overlap) MOKB_TRY(get_async(&as));
     cudaStream_t s_in = overlap ? as->s1 : stream;
-    cudaStream_t s_q = overlap ? as->s2 : stream;
-    const int comm_blocks = overlap ? a->num_comm_sms * kCommBlocksPerSm : 0;
+    const int comm_blocks = overlap ? quant_comm_block_count(a->num_comm_sms) : 0;
     // recompute only rebuilds macrobatch 0 (the saved context); the forward walks all of them, last first
     const int n_macro = with_down ? macrobatches(C, MB) : 1;
     const GateUpWeights wgu{a->w_routed_gate, a->w_routed_gate_sc, a->w_routed_up, a->w_routed_up_sc};
 
     MOKB_TRY(run_prologue(a->tokens_per_expert, a->num_tokens, a->peer_rank, E_l, C, MB, T, s, a->status, stream));
     const void* x_local = reinterpret_cast<const void*>(static_cast<uintptr_t>(a->x_ptrs_host[a->ep_rank]));
-    bool shared_done = false;
 
     for (int mi = 0; mi < n_macro; ++mi) {
         const int m = n_macro - 1 - mi;
@@ -135,9 +132,8 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_mxfp8(const mokb_fwd_mxfp8_a
         // only macrobatch 0 (the one that is always populated) is cut into overlap windows, which are tied to the one
         // persistent GEMM launch by counters (layer.cu)
         const int chunk = m == 0 ? chunk_rows_for(MB, a->minibatch_size) : MB;
-        const int nchunks = (hi - lo + chunk - 1) / chunk;
         const bool flags = overlap && m == 0;
-        const FwdView v = fwd_view(lo, H, I, a->x_routed, a->x_fp8, a->x_sc, a->x_fp8_t, a->x_sc_t, a->gate_fp8,
+        const FwdView v = fwd_view(lo, H, I, a->x_fp8, a->x_sc, a->x_fp8_t, a->x_sc_t, a->gate_fp8,
                                    a->gate_sc, a->up_fp8, a->up_sc, a->hidden_fp8, a->hidden_sc, a->hidden_fp8_t, a->hidden_sc_t);
         void* y_r = (with_down && a->y_routed) ? rebase(a->y_routed, lo, 2ull * H) : nullptr;
 
@@ -145,28 +141,15 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_mxfp8(const mokb_fwd_mxfp8_a
             MOKB_CUDA(cudaEventRecord(as->fork, stream));
             MOKB_CUDA(cudaStreamWaitEvent(s_in, as->fork, 0));
         }
-        // dispatch, window by window: the pull also quantises every row along its columns (what the GEMM reads) and
-        // raises the window's counter; the token-wise form (for the weight gradients of the backward pass) follows
-        // from the bf16 rows on a second, lower-priority side stream, window by window behind the pull, under the GEMM
-        for (int c = 0; c < nchunks; ++c) {
-            const int r0 = lo + c * chunk, r1 = r0 + chunk < hi ? r0 + chunk : hi;
-            MOKB_TRY(dispatch_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, r0, r1, a->topk, H,
-                                        v.x_routed, nullptr, nullptr, comm_blocks, s_in, flags ? s.win_ready + c : nullptr,
-                                        v.x_fp8, v.x_sc, routes, a->status));
-            if (overlap) {
-                MOKB_CUDA(cudaEventRecord(as->ev_in[c], s_in));
-                MOKB_CUDA(cudaStreamWaitEvent(s_q, as->ev_in[c], 0));
-            }
-            MOKB_TRY(quantize_impl(v.x_routed, 1, MB, H, s.n_rows, r0, r1, nullptr, nullptr, v.x_fp8_t, v.x_sc_t, s_q, comm_blocks));
-        }
-        if (overlap) {
-            MOKB_CUDA(cudaEventRecord(as->join1, s_in));
-            MOKB_CUDA(cudaEventRecord(as->join2, s_q));
-        }
+        // dispatch, in row order: the pull quantises every row along its columns (what the GEMM reads) and along tokens
+        // (for the weight gradients of the backward pass) and counts the rows that have arrived, window by window
+        MOKB_TRY(pull_quant_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
+                                      nullptr, nullptr, v.x_fp8, v.x_sc, v.x_fp8_t, v.x_sc_t, MB, comm_blocks, s_in,
+                                      flags ? s.ticket : nullptr, s.win_ready, chunk, routes, a->status));
+        if (overlap) MOKB_CUDA(cudaEventRecord(as->join1, s_in));
 
-        if (!shared_done) {
-            // shared expert (BF16): gate/up + SwiGLU in one pass, then down (independent of the dispatch)
-            shared_done = true;
+        if (m == 0) {
+            // shared expert (BF16): gate/up + SwiGLU in one pass, then down, under macrobatch 0's dispatch
             mokb_gemm_args g = gemm_base(a->status);
             g.mode = 1; g.rows_static = T; g.N = I; g.K = H;
             g.A = x_local; g.lda = H; g.B = a->w_shared_gate; g.B2 = a->w_shared_up; g.ldb = H;
@@ -193,7 +176,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_mxfp8(const mokb_fwd_mxfp8_a
         f.t_rows = MB; f.has_swiglu_limit = a->has_swiglu_limit; f.swiglu_limit = a->swiglu_limit;
         f.window_rows = chunk;
         f.blk_done = s.blk_done + lo / 256;
-        if (flags) { f.win_ready = s.win_ready; f.win_ready_target = comm_blocks; }
+        if (flags) { f.win_ready = s.win_ready; f.win_ready_target = -pull_quant_arrivals(H); }
         f.ldd = H;
         if (with_down) {
             f.B3 = a->w_routed_down; f.B3_sc = a->w_routed_down_sc; f.N2 = H; f.D = y_r;
@@ -201,10 +184,8 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_mxfp8(const mokb_fwd_mxfp8_a
             f.push_rank = a->peer_rank; f.push_idx = a->peer_token_idx; f.push_index_limit = routes;
         }
         MOKB_TRY(mokb_grouped_gemm_mxfp8(&f, stream));
-        // the next macrobatch (or the caller) reuses the pulled rows: the side stream must be done with them
+        // the next macrobatch (or the caller) reuses the pulled rows, and the token-wise form is an output of this call
         if (flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->join1, 0));
-        // ... and with the token-wise copies, which are outputs of this call (and read the pulled rows)
-        if (overlap) MOKB_CUDA(cudaStreamWaitEvent(stream, as->join2, 0));
     }
     return MOKB_OK;
 }
@@ -221,14 +202,14 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
     MOKB_REQUIRE(a->d_x_shared && a->d_gate_shared && a->d_gate_fp8 && a->d_gate_sc && a->d_up_shared && a->d_up_fp8 &&
                  a->d_up_sc && a->d_hidden_shared && a->d_hidden_routed && a->d_y_fp8 && a->d_y_sc && a->d_w_shared_gate &&
                  a->d_w_routed_gate && a->d_w_shared_up && a->d_w_routed_up && a->d_w_shared_down && a->d_w_routed_down, "bwd_mxfp8: null output");
-    MOKB_REQUIRE(a->d_y_routed && a->d_y_fp8_t && a->d_y_sc_t && a->d_gate_fp8_t && a->d_gate_sc_t && a->d_up_fp8_t && a->d_up_sc_t && a->partials,
+    MOKB_REQUIRE(a->d_y_fp8_t && a->d_y_sc_t && a->d_gate_fp8_t && a->d_gate_sc_t && a->d_up_fp8_t && a->d_up_sc_t && a->partials,
                  "bwd_mxfp8: null work buffer");
     const int T = a->num_local_tokens, H = a->hidden, I = a->intermediate, E_l = a->num_local_experts, MB = a->macrobatch_size;
     const int C = a->schedule_capacity;
     const int64_t routes = static_cast<int64_t>(T) * a->topk;      // every rank's routes are numbered [0, routes)
     const int n_macro = macrobatches(C, MB);
     if (n_macro > 1)
-        MOKB_REQUIRE(a->w_routed_gate && a->w_routed_gate_sc && a->w_routed_up && a->w_routed_up_sc && a->x_routed && a->x_fp8 && a->x_sc &&
+        MOKB_REQUIRE(a->w_routed_gate && a->w_routed_gate_sc && a->w_routed_up && a->w_routed_up_sc && a->x_fp8 && a->x_sc &&
                      a->hidden_fp8 && a->hidden_sc,
                      "bwd_mxfp8: schedule_capacity > macrobatch_size needs the forward weights and the replay work buffers");
     const Scratch s = carve(a->scratch, C, E_l, MB);
@@ -236,7 +217,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
     Async* as = nullptr;
     if (overlap) MOKB_TRY(get_async(&as));
     cudaStream_t s_in = overlap ? as->s1 : stream;
-    const int comm_blocks = overlap ? a->num_comm_sms * kCommBlocksPerSm : 0;
+    const int comm_blocks = overlap ? quant_comm_block_count(a->num_comm_sms) : 0;
     const int lim = a->has_swiglu_limit;
     const float limv = a->swiglu_limit;
     const GateUpWeights wgu{a->w_routed_gate, a->w_routed_gate_sc, a->w_routed_up, a->w_routed_up_sc};
@@ -248,9 +229,8 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
     for (int m = 0; m < n_macro; ++m) {
         const int lo = m * MB, hi = (lo + MB < C) ? lo + MB : C;
         // the context (macrobatch 0: as saved; later ones: rebuilt below) and the work buffers, addressed by schedule row
-        const FwdView v = fwd_view(lo, H, I, a->x_routed, a->x_fp8, a->x_sc, a->x_fp8_t, a->x_sc_t, a->gate_fp8,
+        const FwdView v = fwd_view(lo, H, I, a->x_fp8, a->x_sc, a->x_fp8_t, a->x_sc_t, a->gate_fp8,
                                    a->gate_sc, a->up_fp8, a->up_sc, a->hidden_fp8, a->hidden_sc, a->hidden_fp8_t, a->hidden_sc_t);
-        void* d_y_r = rebase(a->d_y_routed, lo, 2ull * H);
         void* d_y_fp8 = rebase(a->d_y_fp8, lo, 1ull * H);
         void* d_y_sc = rebase_scales(a->d_y_sc, lo, H);
         void* d_y_fp8_t = rebase_t(a->d_y_fp8_t, lo);
@@ -273,29 +253,19 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
             MOKB_CUDA(cudaEventRecord(as->fork, stream));
             MOKB_CUDA(cudaStreamWaitEvent(s_in, as->fork, 0));
         }
-        if (m > 0) {       // replay: pull x again and quantise it both ways
-            MOKB_TRY(dispatch_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
-                                        v.x_routed, nullptr, nullptr, comm_blocks, s_in, nullptr, v.x_fp8, v.x_sc, routes, a->status));
-            MOKB_TRY(quantize_impl(v.x_routed, 1, MB, H, s.n_rows, lo, hi, nullptr, nullptr, v.x_fp8_t, v.x_sc_t, s_in, comm_blocks));
-        }
+        if (m > 0)         // replay: pull x again and quantise it both ways
+            MOKB_TRY(pull_quant_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
+                                          nullptr, nullptr, v.x_fp8, v.x_sc, v.x_fp8_t, v.x_sc_t, MB, comm_blocks, s_in, nullptr, nullptr, 0,
+                                          routes, a->status));
         if (overlap) MOKB_CUDA(cudaEventRecord(as->join1, s_in));     // the replayed x is in place
-        // reverse combine: pull d_y rows scaled by the route's router weight and quantise them both ways, in a few windows
-        // (macrobatch 0: the pull's blocks raise the window's counter for the one d_hidden launch below)
+        // reverse combine: pull d_y rows scaled by the route's router weight and quantise them both ways (macrobatch 0: in
+        // row order, counting the rows that have arrived for the one d_hidden launch below)
         const bool flags = overlap && m == 0;
-        const int bchunk = bwd_chunk_rows(hi - lo, m == 0);
-        const int nb = (hi - lo + bchunk - 1) / bchunk;
-        for (int c = 0; c < nb; ++c) {
-            const int r0 = lo + c * bchunk, r1 = r0 + bchunk < hi ? r0 + bchunk : hi;
-            MOKB_TRY(dispatch_rows_impl(a->d_y_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, r0, r1, a->topk, H,
-                                        d_y_r, a->router_weight_ptrs_host, w_row, comm_blocks, s_in, flags ? s.win_ready + c : nullptr,
-                                        d_y_fp8, d_y_sc, routes, a->status));
-        }
-        if (overlap) MOKB_CUDA(cudaEventRecord(as->ev_in[0], s_in));
-        for (int c = 0; c < nb; ++c) {       // the token-wise form of d_y, for the weight gradients at the end
-            const int r0 = lo + c * bchunk, r1 = r0 + bchunk < hi ? r0 + bchunk : hi;
-            MOKB_TRY(quantize_impl(d_y_r, 1, MB, H, s.n_rows, r0, r1, nullptr, nullptr, d_y_fp8_t, d_y_sc_t, s_in, comm_blocks));
-        }
-        if (overlap) MOKB_CUDA(cudaEventRecord(as->ev_in[1], s_in));
+        const int chunk = chunk_rows_for(MB, a->minibatch_size);
+        MOKB_TRY(pull_quant_rows_impl(a->d_y_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
+                                      a->router_weight_ptrs_host, w_row, d_y_fp8, d_y_sc, d_y_fp8_t, d_y_sc_t, MB, comm_blocks, s_in,
+                                      flags ? s.ticket : nullptr, s.win_ready, chunk, routes, a->status));
+        if (overlap) MOKB_CUDA(cudaEventRecord(as->join2, s_in));
 
         if (m == 0) {
             // ---- shared expert (BF16; overlaps the dispatch above)
@@ -326,14 +296,14 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
         if (m > 0)         // replay gate|up + SwiGLU + quantisation into the context buffers
             MOKB_TRY(gate_up_swiglu(v, wgu, s, lo, hi, hi, MB, E_l, H, I, lim, limv, a->status, stream));
         // d_hidden = d_y_q * WdT_q^T: one launch, window by window behind the pull
-        if (overlap && !flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->ev_in[0], 0));
+        if (overlap && !flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->join2, 0));
         mokb_gemm_fp8_args f = fp8_base(a->status);
         f.mode = 0; f.rows_static = hi; f.row_begin = lo; f.row_end = hi;
         f.num_rows = s.n_rows; f.group_of_block = s.group_of_block; f.G = E_l; f.N = I; f.K = H;
         f.A = d_y_fp8; f.A_sc = d_y_sc; f.B = a->w_routed_down_t; f.B_sc = a->w_routed_down_t_sc; f.D = d_hidden_r; f.ldd = I;
-        if (flags) { f.window_rows = bchunk; f.win_ready = s.win_ready; f.win_ready_target = comm_blocks; }
+        if (flags) { f.window_rows = chunk; f.win_ready = s.win_ready; f.win_ready_target = -pull_quant_arrivals(H); }
         MOKB_TRY(mokb_grouped_gemm_mxfp8(&f, stream));
-        if (flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->ev_in[0], 0));
+        if (flags) MOKB_CUDA(cudaStreamWaitEvent(stream, as->join2, 0));
         MOKB_TRY(swiglu_bwd_quant_impl(v.gate_fp8, v.gate_sc, v.up_fp8, v.up_sc, d_hidden_r, MB, I, s.n_rows, lo, hi, lim, limv, w_row,
                                        d_gate_fp8, d_gate_sc, d_gate_fp8_t, d_gate_sc_t, d_up_fp8, d_up_sc, d_up_fp8_t, d_up_sc_t,
                                        partials, d_w_row, stream));
@@ -359,7 +329,6 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
         // the token-wise tensors are passed as they lie in memory ([., MB], first token column = lo)
         MOKB_TRY(wgrad_fp8(a->d_gate_fp8_t, a->d_gate_sc_t, I, a->x_fp8_t, a->x_sc_t, H, a->d_w_routed_gate));
         MOKB_TRY(wgrad_fp8(a->d_up_fp8_t, a->d_up_sc_t, I, a->x_fp8_t, a->x_sc_t, H, a->d_w_routed_up));
-        if (overlap) MOKB_CUDA(cudaStreamWaitEvent(stream, as->ev_in[1], 0));      // the token-wise d_y is complete
         MOKB_TRY(wgrad_fp8(a->d_y_fp8_t, a->d_y_sc_t, H, a->hidden_fp8_t, a->hidden_sc_t, I, a->d_w_routed_down));
     }
     return MOKB_OK;

@@ -128,6 +128,8 @@ _sig("mokb_combine_rows", c_int, c_vp, c_u64p, c_int, c_vp, c_vp, c_vp, c_int, c
 _sig("mokb_comm_default_blocks", c_int)
 _sig("mokb_dispatch_rows_window", c_int, c_u64p, c_int, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int, c_i64, c_vp, c_u64p, c_vp, c_int,
      c_vp, c_vp, c_vp, c_i64, c_vp, c_vp)
+_sig("mokb_dispatch_rows_quant", c_int, c_u64p, c_int, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int, c_i64, c_u64p, c_vp, c_vp, c_vp, c_vp, c_vp,
+     c_i64, c_int, c_vp, c_vp, c_int, c_i64, c_vp, c_vp)
 _sig("mokb_combine_rows_window", c_int, c_vp, c_u64p, c_int, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_i64, c_vp, c_u64p, c_int, c_vp,
      c_int, c_vp, c_i64, c_vp)
 _sig("mokb_swiglu_fwd", c_int, c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_int, c_f32, c_vp)
@@ -140,7 +142,7 @@ EXPORTED = [
     "mokb_mxfp8_quantize", "mokb_fwd_epilogue", "mokb_bwd_epilogue", "mokb_layer_scratch_bytes",
     "mokb_dispatch_mlp_swiglu_combine_fwd_bf16", "mokb_dispatch_mlp_swiglu_combine_bwd_bf16",
     "mokb_grouped_gemm_bf16", "mokb_grouped_gemm_mxfp8", "mokb_dispatch_rows", "mokb_combine_rows", "mokb_swiglu_fwd", "mokb_swiglu_bwd",
-    "mokb_comm_default_blocks", "mokb_dispatch_rows_window", "mokb_combine_rows_window",
+    "mokb_comm_default_blocks", "mokb_dispatch_rows_window", "mokb_dispatch_rows_quant", "mokb_combine_rows_window",
 ]
 
 
@@ -585,6 +587,16 @@ def dispatch_rows_window(src_ptrs, peer_rank, peer_token_idx, num_rows, max_rows
                                       None if row_scale_ptrs is None else _ptr_array(row_scale_ptrs), _p(row_scale_out),
                                       blocks, _p(done_counter), _p(q_out), _p(q_sc_out), index_limit,
                                       _p(status_tensor(dst.device)), _stream()))
+
+
+def dispatch_rows_quant(src_ptrs, peer_rank, peer_token_idx, num_rows, max_rows, row_divisor, hidden, q, sc, qt, sct, *,
+                        row_scale_ptrs=None, row_scale_out=None, blocks=0, ticket=None, window_ready=None, window_rows=0,
+                        index_limit=0):
+    _ck(lib.mokb_dispatch_rows_quant(_ptr_array(src_ptrs), len(src_ptrs), _p(peer_rank), _p(peer_token_idx), _p(num_rows),
+                                     max_rows, 0, max_rows, row_divisor, hidden,
+                                     None if row_scale_ptrs is None else _ptr_array(row_scale_ptrs), _p(row_scale_out),
+                                     _p(q), _p(sc), _p(qt), _p(sct), qt.shape[1], blocks, _p(ticket), _p(window_ready), window_rows,
+                                     index_limit, _p(status_tensor(q.device)), _stream()))
 
 
 def combine_rows_window(src, dst_ptrs, peer_rank, peer_token_idx, num_rows, max_rows, row_begin, row_end, hidden,

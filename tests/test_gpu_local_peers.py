@@ -174,6 +174,42 @@ def test_dispatch_quantises_the_rows_it_pulls_like_the_quantiser(R, T, K, H, sca
     assert int((torch.from_numpy(pr[:N]) < 0).sum()) > 0          # the case has padding rows
 
 
+@pytest.mark.parametrize("R,T,K,H,scaled,window", [(2, 512, 2, 256, False, 256), (4, 512, 4, 512, True, 0), (2, 512, 2, 7168, True, 512)])
+def test_the_quantising_pull_matches_the_pull_and_the_quantiser(R, T, K, H, scaled, window):
+    """Both MXFP8 forms straight from the pulled registers against the bf16 pull followed by the two-way quantiser: bytes and
+    scales identical, padding rows included; by ticket also the count of arrivals per window."""
+    from mok import _C, ops
+    E_l = 2
+    routes = make_routes(R, T, K, E_l, seed=95 + R)
+    g = torch.Generator().manual_seed(96)
+    x = [(torch.randn(T, H, generator=g) * torch.exp(torch.randn(T, 1, generator=g) * 2)).to(torch.bfloat16).cuda() for _ in range(R)]
+    w = [torch.rand(T, K, generator=g).cuda() for _ in range(R)]
+    C = T * K * R
+    pr, pt, nt, tpe = O.schedule(routes, E_l, C, R - 1)
+    N = int(nt[0])
+    prd, ptd, ntd = (torch.from_numpy(a).cuda() for a in (pr, pt, nt))
+    xs, ws = [t.data_ptr() for t in x], [t.data_ptr() for t in w] if scaled else None
+    rows = torch.zeros(C, H, dtype=torch.bfloat16, device="cuda")
+    want_w, got_w = (torch.full((C,), -1.0, device="cuda") if scaled else None for _ in range(2))
+    _C.dispatch_rows(xs, prd, ptd, ntd, C, K, H, rows, ws, want_w)
+    want = ops.mxfp8_quantize(rows[:N].contiguous(), True, True)
+    u8 = dict(dtype=torch.uint8, device="cuda")
+    q, sc = torch.zeros(C, H, **u8), torch.zeros(C // 128, H // 128, 32, 16, **u8)
+    qt, sct = torch.zeros(H, C, **u8), torch.zeros(H // 128, C // 128, 32, 16, **u8)
+    ready = torch.zeros(C // (window or C) + 1, dtype=torch.int32, device="cuda")
+    extra = dict(ticket=torch.zeros(1, dtype=torch.int32, device="cuda"), window_ready=ready, window_rows=window) if window else {}
+    _C.dispatch_rows_quant(xs, prd, ptd, ntd, C, K, H, q, sc, qt, sct, row_scale_ptrs=ws, row_scale_out=got_w, blocks=16, index_limit=T * K, **extra)
+    torch.cuda.synchronize()
+    assert _C.check_status() == 0
+    assert torch.equal(q[:N], want[0].view(torch.uint8)) and torch.equal(sc[:N // 128], want[1])
+    assert torch.equal(qt[:, :N], want[2].view(torch.uint8)) and torch.equal(sct[:, :N // 128], want[3])
+    assert not q[N:].any() and not qt[:, N:].any()
+    assert not scaled or torch.equal(got_w[:N], want_w[:N])
+    if window:
+        assert ready.tolist() == [max(0, min(N, (c + 1) * window) - c * window) // 256 * (H // 32) for c in range(ready.numel())]
+    assert int((torch.from_numpy(pr[:N]) < 0).sum()) > 0          # the case has padding rows
+
+
 def test_transposed_only_quantiser_matches_the_two_way_quantiser():
     from mok import ops
     g = torch.Generator().manual_seed(92)
