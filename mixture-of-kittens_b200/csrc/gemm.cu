@@ -213,12 +213,9 @@ __device__ __forceinline__ void st_global_v4(void* p, uint32_t a, uint32_t b, ui
     asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
-// 32 fp32 accumulator columns of one row -> 32 bf16 (64 bytes) in global memory; `wide`: the row is 32-byte
-// aligned, so two 32-byte stores (one full sector each) replace four 16-byte ones
-__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (&r)[32], bool wide) {
-    uint32_t w[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) w[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+// 32 bf16 columns of one row (64 bytes) to global memory; `wide`: the row is 32-byte aligned, so two 32-byte stores (one
+// full sector each) replace four 16-byte ones
+__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (&w)[16], bool wide) {
     if (wide) {
 #pragma unroll
         for (int q = 0; q < 2; ++q)
@@ -228,6 +225,61 @@ __device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (
     } else {
 #pragma unroll
         for (int q = 0; q < 4; ++q) st_global_v4(dst + 8 * q, w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+    }
+}
+// the same from fp32 accumulator columns
+__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (&r)[32], bool wide) {
+    uint32_t w[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+    store_row32(dst, w, wide);
+}
+
+// 32 gate and up columns of this warp's rows from tensor memory (rounded to bf16, as pairs) and hidden = silu(gate) * up of the
+// rounded values, clamped at `limit` (infinity: not).  The quotient is a reciprocal and a product: its two units in the last
+// place of fp32 are below what __expf leaves, and the IEEE division's branch kept the 32 columns from overlapping.
+__device__ __forceinline__ void load_32_columns(uint32_t taddr, uint32_t (&w)[16]) {
+    uint32_t r[32];
+    tmem_ld_32x32(taddr, r);
+    tmem_ld_wait_for(r);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+}
+__device__ __forceinline__ void swiglu_32_columns(uint32_t t_gate, uint32_t t_up, float limit, uint32_t (&gw)[16], uint32_t (&uw)[16],
+                                                  uint32_t (&hw)[16]) {
+    load_32_columns(t_gate, gw);
+    load_32_columns(t_up, uw);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        float2 gf = unpack_bf16(gw[i]), uf = unpack_bf16(uw[i]);
+        if (limit < __int_as_float(0x7f800000)) {
+            gf.x = fminf(gf.x, limit);
+            gf.y = fminf(gf.y, limit);
+            uf.x = fminf(fmaxf(uf.x, -limit), limit);
+            uf.y = fminf(fmaxf(uf.y, -limit), limit);
+        }
+        hw[i] = pack_bf16(__fdividef(gf.x, 1.0f + __expf(-gf.x)) * uf.x, __fdividef(gf.y, 1.0f + __expf(-gf.y)) * uf.y);
+    }
+}
+
+// A warp's 32 rows x 64 bf16 columns through a 4 KB shared-memory buffer: lane = row stages 32 columns at a time (16-byte
+// unit u of a row at position u ^ (row & 7): conflict-free both ways), then eight lanes store one whole 128-byte line of a row
+// and a store instruction touches 4 lines instead of 32 sectors of 32 different lines.
+__device__ __forceinline__ void stage_32_columns(uint32_t stage, int lane, int half, const uint32_t (&w)[16]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + lane * 128u + static_cast<uint32_t>(((4 * half + u) ^ (lane & 7)) << 4)),
+                     "r"(w[4 * u]), "r"(w[4 * u + 1]), "r"(w[4 * u + 2]), "r"(w[4 * u + 3]) : "memory");
+}
+__device__ __forceinline__ void store_lines(uint32_t stage, int lane, __nv_bfloat16* dst, int ld) {
+    const int sub = lane >> 3, unit = lane & 7;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int rr = 4 * i + sub;
+        uint32_t v0, v1, v2, v3;
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
+                     : "r"(stage + rr * 128u + static_cast<uint32_t>((unit ^ (rr & 7)) << 4)) : "memory");
+        st_global_v4(dst + static_cast<size_t>(rr) * ld + unit * 8, v0, v1, v2, v3);
     }
 }
 
@@ -450,28 +502,45 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             if (MODE == MODE_SWIGLU || (MODE == MODE_FWD && ti.phase == 0)) {
                 const size_t row = static_cast<size_t>(ti.m_blk) * G::TILE_M + row_in_tile;
                 const size_t off = row * p.ldd + static_cast<size_t>(ti.n_blk) * 128;
+                const float limit = p.has_limit ? p.limit : __int_as_float(0x7f800000);
+                if (p.line_stores) {
+                    // 64 columns at a time of gate, up and hidden go through the warp's 4 KB buffer one after the other and
+                    // leave as whole 128-byte lines
+                    const uint32_t stage = bars + 256u + static_cast<uint32_t>(warp - 2) * 4096u;
+                    const size_t warp_off = off - static_cast<size_t>(lane) * p.ldd;
 #pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
-                    uint32_t g[32], u[32];
-                    tmem_ld_32x32(t_addr + c * 32, g);
-                    tmem_ld_32x32(t_addr + 128 + c * 32, u);
-                    tmem_ld_wait();
-                    uint32_t h[32];
+                    for (int cp = 0; cp < 2; ++cp) {
+                        uint32_t uw[2][16], hw[2][16];
+                        __syncwarp();             // the previous tensor has been read out of the buffer
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float gf = bf16_round(__uint_as_float(g[i]));
-                        float uf = bf16_round(__uint_as_float(u[i]));
-                        g[i] = __float_as_uint(gf);
-                        u[i] = __float_as_uint(uf);
-                        if (p.has_limit) {
-                            gf = fminf(gf, p.limit);
-                            uf = fminf(fmaxf(uf, -p.limit), p.limit);
+                        for (int half = 0; half < 2; ++half) {
+                            uint32_t gw[16];
+                            swiglu_32_columns(t_addr + cp * 64 + half * 32, t_addr + 128 + cp * 64 + half * 32, limit, gw, uw[half], hw[half]);
+                            stage_32_columns(stage, lane, half, gw);
                         }
-                        h[i] = __float_as_uint(gf / (1.0f + __expf(-gf)) * uf);
+                        const size_t at = warp_off + cp * 64;
+                        __syncwarp();
+                        store_lines(stage, lane, p.D + at, p.ldd);
+                        __syncwarp();
+                        stage_32_columns(stage, lane, 0, uw[0]);
+                        stage_32_columns(stage, lane, 1, uw[1]);
+                        __syncwarp();
+                        store_lines(stage, lane, p.D2 + at, p.ldd);
+                        __syncwarp();
+                        stage_32_columns(stage, lane, 0, hw[0]);
+                        stage_32_columns(stage, lane, 1, hw[1]);
+                        __syncwarp();
+                        store_lines(stage, lane, p.D3 + at, p.ldd);
                     }
-                    store_row32(p.D + off + c * 32, g, p.wide_stores);
-                    store_row32(p.D2 + off + c * 32, u, p.wide_stores);
-                    store_row32(p.D3 + off + c * 32, h, p.wide_stores);
+                } else {
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t gw[16], uw[16], hw[16];
+                        swiglu_32_columns(t_addr + c * 32, t_addr + 128 + c * 32, limit, gw, uw, hw);
+                        store_row32(p.D + off + c * 32, gw, p.wide_stores);
+                        store_row32(p.D2 + off + c * 32, uw, p.wide_stores);
+                        store_row32(p.D3 + off + c * 32, hw, p.wide_stores);
+                    }
                 }
             } else {
                 const int tile_row = ti.m_blk * G::TILE_M + row_in_tile;
