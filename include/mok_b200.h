@@ -303,7 +303,8 @@ int mokb_struct_sizes_mxfp8(int* out, int n);
  *   mode 1: same as 0 with B = gate and B2 = up   -> D = gate, D2 = up, D3 = SwiGLU(gate, up), all [rows, N]
  *   mode 2: B [G, K, N] (N contiguous; "dgrad")   -> D [rows, N]; if A2/B2 given, D = A*B + A2*B2
  * Weight-gradient GEMM (mode 3): for each group g with rows [off[g], off[g+1]) of
- * A [rows, M] and B [rows, N]: D[g] [M, N] = A_g^T * B_g (zero if the group is empty).
+ * A [rows, M] and B [rows, N]: D[g] [M, N] = A_g^T * B_g (zero if the group is empty).  With A2 [rows, N], B2 [rows, M] and
+ * B3 [rows, N] (contiguous): also D2[g] [N, M] = A2_g^T * B2_g and D3[g] [N, M] = B3_g^T * B2_g in the same launch.
  *   mode 4: mode 1 followed by the down projection of the same rows, D4 [rows, N2] = D3 * B3[g]^T with B3 [G, N2, N],
  *           in ONE persistent launch that walks the rows in order, the down tiles a few super-groups of 1024 rows behind the
  *           gate/up tiles (windows long enough: all gate/up tiles of a window, then all its down tiles -- the task order of
@@ -375,7 +376,8 @@ int mokb_grouped_gemm_bf16(const mokb_gemm_args* args, void* stream);
  *           t_first: A and B hold the token columns [t_first, t_first + rows_static) of the row space that
  *           group_offsets refers to (a macrobatch of a longer schedule); offsets outside are not allowed.
  *           accumulate != 0 adds to the stored bf16 D (a group with an empty window then leaves D untouched
- *           instead of zeroing it).
+ *           instead of zeroing it).  With A2 (and B2, B3, D2, D3): also D2[g][N,M] = A2[N, cols_g] * B2[M, cols_g]^T and
+ *           D3[g][N,M] = B3[N, cols_g] * B2[M, cols_g]^T in the same launch.
  *   mode 3: the two products of mode 1 without the bf16 round trip: gate and up are rounded to bf16 in the
  *           epilogue, hidden = SwiGLU(gate, up) (clamped if has_swiglu_limit), and the kernel writes gate_q, up_q,
  *           hid_q [rows, N] E4M3 with scales along columns and hid_qt [N, t_rows] with scales along tokens: what
@@ -420,6 +422,7 @@ typedef struct {
     int reserve_sms;
     /* mode 2, optional, device [G]: as in mokb_gemm_args, in steps of 128 tokens */
     const int32_t* group_k_end;
+    void* D3;                       /* mode 2: see there */
 } mokb_gemm_fp8_args;
 int mokb_grouped_gemm_mxfp8(const mokb_gemm_fp8_args* args, void* stream);
 

@@ -75,6 +75,7 @@ int dispatch_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32_t
                        float* row_scale_out, int blocks, cudaStream_t s, int32_t* done_counter = nullptr,
                        void* q_out = nullptr, void* q_sc_out = nullptr, int64_t index_limit = 0, int32_t* status = nullptr,
                        int32_t* ticket = nullptr, int window_rows = 0);
+bool gemm_uses_pairs();          // gemm.cu: the BF16 GEMM runs on CTA pairs (always, except with MOKB_GEMM_CTAS=1)
 int pull_quant_arrivals(int64_t hidden);
 int pull_quant_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32_t* peer_rank, const int32_t* peer_token_idx,
                          const int32_t* num_rows, int max_rows, int row_begin, int row_end, int row_divisor, int64_t hidden,

@@ -24,7 +24,10 @@
 //   MODE_NT      D[rows,N] = A[rows,K] * W[g][N,K]^T                 (down projection)
 //   MODE_SWIGLU  gate,up = A * Wg[g]^T, A * Wu[g]^T; hidden = SwiGLU  (one 128+128 column tile)
 //   MODE_NN      D[rows,N] = A[rows,K] * W[g][K,N] (+ A2 * W2[g])    (input gradients)
-//   MODE_WGRAD   D[g][M,N] = A[rows_g,M]^T * B[rows_g,N]             (weight gradients)
+//   MODE_WGRAD   D[g][M,N] = A[rows_g,M]^T * B[rows_g,N]             (weight gradients), optionally in the same launch also
+//                D2[g][N,M] = A2^T * B2 and D3[g][N,M] = B3^T * B2 over the same rows: an expert's three gradients.  One
+//                launch has one partly filled last wave instead of three, which is what bounds a single expert over many rows
+//                (the shared one: 2048 x 7168 are 224 tiles on 74 CTA pairs, 3.03 waves each but 9.08 together).
 //   MODE_FWD     MODE_SWIGLU tiles and the MODE_NT (down) tiles of the same rows in ONE persistent launch,
 //                the down tiles some super-groups of rows behind: the task loop of the
 //                reference's forward megakernel (csrc/megakernel/forward.cuh:146-266) with its global-memory
@@ -82,6 +85,7 @@ struct KParams {
     int has_limit;
     float limit;
     int accumulate;                  // MODE_WGRAD: add to the stored bf16 result instead of overwriting it
+    int products;                    // MODE_WGRAD: 1 or 3
     // counters (see the top of the file)
     int window_rows;                 // rows per window, a multiple of 256; 0 = one window
     const int32_t* win_ready;        // [windows from row_begin], optional
@@ -106,7 +110,7 @@ struct KParams {
 
 struct Tile {
     int m_blk, n_blk, group, k_iters, k_row0;
-    int phase;                       // MODE_FWD: 0 = gate/up + SwiGLU tile, 1 = down tile
+    int phase;                       // MODE_FWD: 0 = gate/up + SwiGLU tile, 1 = down tile; MODE_WGRAD: which product
     int window;                      // window of the tile's rows, counted from row_begin
 };
 
@@ -122,7 +126,7 @@ struct Sched {
         if (MODE == MODE_WGRAD) {
             m_blocks = (p.M + TM - 1) / TM;
             n_blocks = (p.N + BN - 1) / BN;
-            total = p.G * m_blocks * n_blocks;
+            total = p.G * m_blocks * n_blocks * p.products;        // (products 1 and 2 have the blocks of product 0, transposed)
             // accumulating over no rows at all (an empty macrobatch) leaves every gradient as it is: no tiles
             if (p.accumulate && p.group_offsets[p.G] == p.group_offsets[0]) total = 0;
         } else {
@@ -154,10 +158,13 @@ struct Sched {
         Tile ti;
         if (MODE == MODE_WGRAD) {
             const int per = m_blocks * n_blocks;
-            ti.group = t / per;
-            const int rem = t - ti.group * per;
-            ti.n_blk = rem / m_blocks;
-            ti.m_blk = rem - ti.n_blk * m_blocks;
+            const int unit = t / per;                            // an expert's products one after the other: 1 and 2 share an operand
+            ti.group = unit / p.products;
+            ti.phase = unit - ti.group * p.products;
+            const int rem = t - unit * per;
+            const int mb = ti.phase ? n_blocks : m_blocks;
+            ti.n_blk = rem / mb;
+            ti.m_blk = rem - ti.n_blk * mb;
             ti.k_row0 = p.group_offsets[ti.group];
             int k_end = p.group_offsets[ti.group + 1];
             if (p.group_k_end) k_end = min(k_end, max(p.group_k_end[ti.group], ti.k_row0));
@@ -339,7 +346,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             tma_prefetch_desc(&tmB2);
             if (MODE == MODE_NN) tma_prefetch_desc(&tmA2);
         }
-        if (MODE == MODE_FWD && p.N2 > 0) {
+        if (MODE == MODE_WGRAD && p.products > 1) tma_prefetch_desc(&tmB2);
+        if ((MODE == MODE_FWD && p.N2 > 0) || (MODE == MODE_WGRAD && p.products > 1)) {
             tma_prefetch_desc(&tmA2);
             tma_prefetch_desc(&tmB3);
         }
@@ -377,6 +385,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 const Tile ti = next_ti;
                 if (t + tile_stride < sched.total) next_ti = sched.get(p, t + tile_stride);
                 const int row0 = ti.m_blk * G::TILE_M + static_cast<int>(cta) * 128;    // this CTA's rows of A / D
+                const CUtensorMap* const wg_a = ti.phase == 0 ? &tmA : ti.phase == 1 ? &tmA2 : &tmB3;      // MODE_WGRAD
+                const CUtensorMap* const wg_b = ti.phase == 0 ? &tmB : &tmB2;
                 if (MODE != MODE_WGRAD) {
                     // rows that another kernel (or, for a down tile, other CTAs of this one) is still producing
                     bool fenced = false;
@@ -426,9 +436,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     } else {
                         const int krow = ti.k_row0 - p.row_begin + it * BK;
 #pragma unroll
-                        for (int c = 0; c < 2; ++c) tma_tile<NCTA>(a_dst + c * CHUNK_BYTES, &tmA, fb, row0 + 64 * c, krow);
+                        for (int c = 0; c < 2; ++c) tma_tile<NCTA>(a_dst + c * CHUNK_BYTES, wg_a, fb, row0 + 64 * c, krow);
 #pragma unroll
-                        for (int c = 0; c < G::B_COLS / 64; ++c) tma_tile<NCTA>(b_dst + c * CHUNK_BYTES, &tmB, fb, bcol0 + 64 * c, krow);
+                        for (int c = 0; c < G::B_COLS / 64; ++c) tma_tile<NCTA>(b_dst + c * CHUNK_BYTES, wg_b, fb, bcol0 + 64 * c, krow);
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
@@ -546,14 +556,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 const int tile_row = ti.m_blk * G::TILE_M + row_in_tile;
                 bool row_ok = true;
                 size_t row;
+                const int wg_m = ti.phase ? p.N : p.M, wg_n = ti.phase ? p.M : p.N;      // MODE_WGRAD: this product's [M, N]
                 if (MODE == MODE_WGRAD) {
-                    row_ok = tile_row < p.M;
-                    row = static_cast<size_t>(ti.group) * p.M + tile_row;
+                    row_ok = tile_row < wg_m;
+                    row = static_cast<size_t>(ti.group) * wg_m + tile_row;
                 } else {
                     row = static_cast<size_t>(tile_row);
                 }
-                __nv_bfloat16* const base = MODE == MODE_FWD ? p.D4 : p.D;
-                const size_t ld_out = MODE == MODE_FWD ? p.ldd4 : p.ldd;
+                __nv_bfloat16* const base = MODE == MODE_FWD ? p.D4 : MODE == MODE_WGRAD && ti.phase ? (ti.phase == 1 ? p.D2 : p.D3) : p.D;
+                const size_t ld_out = MODE == MODE_FWD ? p.ldd4 : MODE == MODE_WGRAD && ti.phase ? p.M : p.ldd;
                 __nv_bfloat16* dst = base + row * ld_out + static_cast<size_t>(ti.n_blk) * BN;
                 if (base == nullptr) row_ok = false;          // pushed only
                 __nv_bfloat16* pdst = nullptr;                // this row's place in its home rank's buffer
@@ -566,7 +577,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         if (p.push_values && ti.n_blk == 0) static_cast<float*>(p.push_val.p[pr])[slot] = p.push_values[tile_row];
                     }
                 }
-                const int cols_left = (MODE == MODE_FWD ? p.N2 : p.N) - ti.n_blk * BN;
+                const int cols_left = (MODE == MODE_FWD ? p.N2 : MODE == MODE_WGRAD ? wg_n : p.N) - ti.n_blk * BN;
                 const int nchunks = min(BN / 32, (cols_left + 31) / 32);
                 // one 32-column chunk from registers: (optionally add the stored gradient,) round to bf16, store locally
                 // and / or at home
@@ -654,7 +665,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                             uint32_t v0, v1, v2, v3;
                             asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
                                          : "r"(stage + rr * 128u + static_cast<uint32_t>((unit ^ (rr & 7)) << 4)) : "memory");
-                            if (warp_dst && (MODE != MODE_WGRAD || warp_row0 + rr < p.M))
+                            if (warp_dst && (MODE != MODE_WGRAD || warp_row0 + rr < wg_m))
                                 st_global_v4(warp_dst + static_cast<size_t>(rr) * ld_out + col, v0, v1, v2, v3);
                             if ((MODE == MODE_NT || MODE == MODE_NN || MODE == MODE_FWD) && p.push) {
                                 __nv_bfloat16* home = reinterpret_cast<__nv_bfloat16*>(__shfl_sync(0xffffffffu, own_home, rr));
@@ -735,11 +746,14 @@ int ctas_per_tile() {
 
 template <int MODE>
 int dispatch_launch(int ncta, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2, const CUtensorMap& b2,
-                    const KParams& p, int tiles, cudaStream_t stream) {
-    return ncta == 2 ? launch<MODE, 2>(a, b, a2, b2, b, p, tiles, stream) : launch<MODE, 1>(a, b, a2, b2, b, p, tiles, stream);
+                    const CUtensorMap& b3, const KParams& p, int tiles, cudaStream_t stream) {
+    return ncta == 2 ? launch<MODE, 2>(a, b, a2, b2, b3, p, tiles, stream) : launch<MODE, 1>(a, b, a2, b2, b3, p, tiles, stream);
 }
 
 }  // namespace
+
+bool gemm_uses_pairs() { return ctas_per_tile() == 2; }
+
 }  // namespace mokb
 
 using namespace mokb;
@@ -824,7 +838,7 @@ extern "C" int mokb_grouped_gemm_bf16(const mokb_gemm_args* g, void* stream_) {
         MOKB_TRY(make_tmap_2d(&tb, g->B, 2, g->K, static_cast<uint64_t>(g->G) * g->N, 2ull * g->ldb, 64, b_box));
         p.b_rows_per_group = g->N;
         ta2 = ta; tb2 = tb;
-        return dispatch_launch<MODE_NT>(ncta, ta, tb, ta2, tb2, p, m_tiles * (g->N / BN), stream);
+        return dispatch_launch<MODE_NT>(ncta, ta, tb, ta2, tb2, tb, p, m_tiles * (g->N / BN), stream);
     }
     case MODE_SWIGLU: {
         MOKB_REQUIRE(g->K > 0 && g->K % BK == 0 && g->N > 0 && g->N % 128 == 0, "grouped_gemm SWIGLU: K %% 64 and N %% 128 must be 0");
@@ -834,7 +848,7 @@ extern "C" int mokb_grouped_gemm_bf16(const mokb_gemm_args* g, void* stream_) {
         MOKB_TRY(make_tmap_2d(&tb2, g->B2, 2, g->K, static_cast<uint64_t>(g->G) * g->N, 2ull * g->ldb, 64, 128));
         p.b_rows_per_group = g->N;
         ta2 = ta;
-        return dispatch_launch<MODE_SWIGLU>(ncta, ta, tb, ta2, tb2, p, m_tiles * (g->N / 128), stream);
+        return dispatch_launch<MODE_SWIGLU>(ncta, ta, tb, ta2, tb2, tb, p, m_tiles * (g->N / 128), stream);
     }
     case MODE_NN: {
         MOKB_REQUIRE(g->K > 0 && g->K % BK == 0 && g->N > 0 && g->N % 64 == 0, "grouped_gemm NN: K %% 64 and N %% 64 must be 0");
@@ -848,7 +862,7 @@ extern "C" int mokb_grouped_gemm_bf16(const mokb_gemm_args* g, void* stream_) {
             p.dual = 1;
         }
         p.b_rows_per_group = g->K;
-        return dispatch_launch<MODE_NN>(ncta, ta, tb, ta2, tb2, p, m_tiles * ((g->N + BN - 1) / BN), stream);
+        return dispatch_launch<MODE_NN>(ncta, ta, tb, ta2, tb2, tb, p, m_tiles * ((g->N + BN - 1) / BN), stream);
     }
     case MODE_FWD: {
         MOKB_REQUIRE(g->K > 0 && g->K % BK == 0 && g->N > 0 && g->N % 128 == 0, "grouped_gemm FWD: K %% 64 and N %% 128 must be 0");
@@ -886,9 +900,22 @@ extern "C" int mokb_grouped_gemm_bf16(const mokb_gemm_args* g, void* stream_) {
         MOKB_TRY(make_tmap_2d(&ta, g->A, 2, g->M, rows, 2ull * g->lda, 64, 64));
         MOKB_TRY(make_tmap_2d(&tb, g->B, 2, g->N, rows, 2ull * g->ldb, 64, 64));
         ta2 = ta; tb2 = tb;
+        CUtensorMap tb3 = tb;
         const int wg_ncta = ctas_per_tile();     // the weight-gradient tile is over M and N, not over rows
         const int tm = 128 * wg_ncta;
-        return dispatch_launch<MODE_WGRAD>(wg_ncta, ta, tb, ta2, tb2, p, g->G * ((g->M + tm - 1) / tm) * ((g->N + BN - 1) / BN), stream);
+        p.products = 1;
+        if (g->A2) {
+            // A2 and B3 have N columns, B2 has M: [N, M] gradients, stored without gaps
+            MOKB_REQUIRE(g->B2 && g->B3 && g->D2 && g->D3, "grouped_gemm WGRAD: A2, B2, B3, D2 and D3 go together");
+            MOKB_REQUIRE(wg_ncta == 2 && g->N % 128 == 0, "grouped_gemm WGRAD: three products need CTA pairs and N %% 128 == 0");
+            MOKB_REQUIRE(((reinterpret_cast<uintptr_t>(g->D2) | reinterpret_cast<uintptr_t>(g->D3)) & 15) == 0, "grouped_gemm WGRAD: D2, D3 not 16-byte aligned");
+            MOKB_TRY(make_tmap_2d(&ta2, g->A2, 2, g->N, rows, 2ull * g->N, 64, 64));
+            MOKB_TRY(make_tmap_2d(&tb2, g->B2, 2, g->M, rows, 2ull * g->M, 64, 64));
+            MOKB_TRY(make_tmap_2d(&tb3, g->B3, 2, g->N, rows, 2ull * g->N, 64, 64));
+            p.products = 3;
+            p.wide_stores = p.wide_stores && g->M % 16 == 0;
+        }
+        return dispatch_launch<MODE_WGRAD>(wg_ncta, ta, tb, ta2, tb2, tb3, p, g->G * ((g->M + tm - 1) / tm) * ((g->N + BN - 1) / BN) * p.products, stream);
     }
     }
 }

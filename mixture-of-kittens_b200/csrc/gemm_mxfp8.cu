@@ -71,6 +71,8 @@ struct FParams {
     int ldd;
     int wide_stores;                 // D (and D2) rows are 32-byte aligned: the epilogue stores 32 bytes per instruction
     int accumulate;                  // FMODE_WGRAD: add to the stored bf16 result instead of overwriting it
+    int products;                    // FMODE_WGRAD: 1, or 3 (see gemm.cu)
+    __nv_bfloat16* D3;
     int k_tile_origin;               // FMODE_WGRAD: the operands' first token column, in 128-token tiles, in group_offsets' row space
     // FMODE_GATEUP_QUANT outputs: E4M3 [rows, N] + packed scales for gate, up, hidden; hidden also as [N, t_rows]
     uint8_t *gate_q, *gate_sc, *up_q, *up_sc, *hid_q, *hid_sc, *hid_qt, *hid_sct;
@@ -96,7 +98,7 @@ struct FParams {
 
 struct Tile {
     int m_blk, n_blk, group, k_iters, k_tile0;
-    int phase, window;               // FMODE_FWD: 0 = gate/up tile, 1 = down tile; window of the rows, from row_begin
+    int phase, window;               // FMODE_FWD: 0 = gate/up tile, 1 = down tile; window of the rows, from row_begin.  FMODE_WGRAD: which product
 };
 
 template <int MODE>
@@ -110,7 +112,7 @@ struct Sched {
         if (MODE == FMODE_WGRAD) {
             m_blocks = (p.M + TILE_M - 1) / TILE_M;
             n_blocks = (p.N + BN - 1) / BN;
-            total = p.G * m_blocks * n_blocks;
+            total = p.G * m_blocks * n_blocks * p.products;
             // accumulating over no token columns at all (an empty macrobatch) leaves every gradient as it is: no tiles
             if (p.accumulate && p.group_offsets[p.G] == p.group_offsets[0]) total = 0;
         } else {
@@ -140,10 +142,13 @@ struct Sched {
         Tile ti;
         if (MODE == FMODE_WGRAD) {
             const int per = m_blocks * n_blocks;
-            ti.group = t / per;
-            const int rem = t - ti.group * per;
-            ti.n_blk = rem / m_blocks;
-            ti.m_blk = rem - ti.n_blk * m_blocks;
+            const int unit = t / per;
+            ti.group = unit / p.products;
+            ti.phase = unit - ti.group * p.products;
+            const int rem = t - unit * per;
+            const int mb = ti.phase ? n_blocks : m_blocks;
+            ti.n_blk = rem / mb;
+            ti.m_blk = rem - ti.n_blk * mb;
             const int c0 = p.group_offsets[ti.group];
             ti.k_tile0 = c0 / BKB - p.k_tile_origin;
             int k_end = p.group_offsets[ti.group + 1];
@@ -270,9 +275,9 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
         tma_prefetch_desc(&tm.A); tma_prefetch_desc(&tm.B); tma_prefetch_desc(&tm.SA); tma_prefetch_desc(&tm.SB);
         if (kGateUp<MODE> || p.dual) { tma_prefetch_desc(&tm.B2); tma_prefetch_desc(&tm.SB2); }
         if (p.dual) { tma_prefetch_desc(&tm.A2); tma_prefetch_desc(&tm.SA2); }
-        if (MODE == FMODE_FWD) {
+        if (MODE == FMODE_FWD || (MODE == FMODE_WGRAD && p.products > 1)) {
             tma_prefetch_desc(&tm.B2); tma_prefetch_desc(&tm.SB2);
-            if (p.N2 > 0) { tma_prefetch_desc(&tm.A2); tma_prefetch_desc(&tm.SA2); tma_prefetch_desc(&tm.B3); tma_prefetch_desc(&tm.SB3); }
+            if (MODE == FMODE_WGRAD || p.N2 > 0) { tma_prefetch_desc(&tm.A2); tma_prefetch_desc(&tm.SA2); tma_prefetch_desc(&tm.B3); tma_prefetch_desc(&tm.SB3); }
         }
     }
     if (warp == 1) {
@@ -326,11 +331,15 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
                     if (MODE == FMODE_WGRAD) {
                         const int kt = ti.k_tile0 + it;
                         const int brow = ti.n_blk * BN;
-                        tma_load_2d_pair(a_dst, &tm.A, fb, kt * BKB, row0);
-                        tma_load_2d_pair(b_dst, &tm.B, fb, kt * BKB, brow + static_cast<int>(cta) * 128);
-                        tma_load_2d_pair(sfa_dst, &tm.SA, fb, 0, (row0 / 128) * p.a_ktiles + kt);
-                        tma_load_2d_pair(sfa_dst + SF_TILE, &tm.SB, fb, 0, (brow / 128) * p.b_ktiles + kt);
-                        tma_load_2d_pair(sfa_dst + 2 * SF_TILE, &tm.SB, fb, 0, (brow / 128 + 1) * p.b_ktiles + kt);
+                        const CUtensorMap* const a = ti.phase == 0 ? &tm.A : ti.phase == 1 ? &tm.A2 : &tm.B3;
+                        const CUtensorMap* const sa = ti.phase == 0 ? &tm.SA : ti.phase == 1 ? &tm.SA2 : &tm.SB3;
+                        const CUtensorMap* const b = ti.phase == 0 ? &tm.B : &tm.B2;
+                        const CUtensorMap* const sb = ti.phase == 0 ? &tm.SB : &tm.SB2;
+                        tma_load_2d_pair(a_dst, a, fb, kt * BKB, row0);
+                        tma_load_2d_pair(b_dst, b, fb, kt * BKB, brow + static_cast<int>(cta) * 128);
+                        tma_load_2d_pair(sfa_dst, sa, fb, 0, (row0 / 128) * p.a_ktiles + kt);
+                        tma_load_2d_pair(sfa_dst + SF_TILE, sb, fb, 0, (brow / 128) * p.b_ktiles + kt);
+                        tma_load_2d_pair(sfa_dst + 2 * SF_TILE, sb, fb, 0, (brow / 128 + 1) * p.b_ktiles + kt);
                     } else if (MODE == FMODE_FWD && ti.phase == 1) {
                         const int brow = ti.group * p.b3_rows_per_group + ti.n_blk * BN;
                         tma_load_2d_pair(a_dst, &tm.A2, fb, it * BKB, row0);
@@ -497,12 +506,16 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
             if (MODE == FMODE_DUALB) {
                 dst = (half ? p.D2 : p.D) + row * p.ldd + static_cast<size_t>(ti.n_blk) * 128;
             } else {
+                __nv_bfloat16* base = p.D;
+                int ld_out = p.ldd, n_cols = MODE == FMODE_FWD ? p.N2 : p.N;
                 if (MODE == FMODE_WGRAD) {
-                    row_ok = tile_row < p.M;
-                    row += static_cast<size_t>(ti.group) * p.M;
+                    const int wg_m = ti.phase ? p.N : p.M;               // this product's rows
+                    if (ti.phase) { base = ti.phase == 1 ? p.D2 : p.D3; ld_out = n_cols = p.M; }
+                    row_ok = tile_row < wg_m;
+                    row += static_cast<size_t>(ti.group) * wg_m;
                 }
-                dst = p.D + row * p.ldd + static_cast<size_t>(ti.n_blk) * BN + half * 128;
-                cols_left = (MODE == FMODE_FWD ? p.N2 : p.N) - ti.n_blk * BN - half * 128;
+                dst = base + row * ld_out + static_cast<size_t>(ti.n_blk) * BN + half * 128;
+                cols_left = n_cols - ti.n_blk * BN - half * 128;
                 if (p.D == nullptr) row_ok = false;        // pushed only
             }
             __nv_bfloat16* pdst = nullptr;                 // this row's place in its home rank's buffer
@@ -717,7 +730,20 @@ extern "C" int mokb_grouped_gemm_mxfp8(const mokb_gemm_fp8_args* g, void* stream
         p.a_ktiles = p.b_ktiles = static_cast<int>(rows / 128);
         p.k_tile_origin = g->t_first / BKB;
         p.accumulate = g->accumulate;
-        return launch<FMODE_WGRAD>(m, p, g->G * ((g->M + TILE_M - 1) / TILE_M) * ((g->N + BN - 1) / BN), stream);
+        p.products = 1;
+        if (g->A2) {
+            MOKB_REQUIRE(g->A2_sc && g->B2 && g->B2_sc && g->B3 && g->B3_sc && g->D2 && g->D3, "grouped_gemm_mxfp8 WGRAD: A2, B2, B3 (data and scales), D2 and D3 go together");
+            MOKB_TRY(data_map(&m.A2, g->A2, rows, g->N));
+            MOKB_TRY(data_map(&m.B3, g->B3, rows, g->N));
+            MOKB_TRY(data_map(&m.B2, g->B2, rows, g->M));
+            MOKB_TRY(scale_map(&m.SA2, g->A2_sc, static_cast<uint64_t>(g->N / 128) * (rows / 128)));
+            MOKB_TRY(scale_map(&m.SB3, g->B3_sc, static_cast<uint64_t>(g->N / 128) * (rows / 128)));
+            MOKB_TRY(scale_map(&m.SB2, g->B2_sc, static_cast<uint64_t>(g->M / 128) * (rows / 128)));
+            p.products = 3;
+            p.D3 = static_cast<__nv_bfloat16*>(g->D3);
+            p.wide_stores = p.wide_stores && g->M % 16 == 0 && reinterpret_cast<uintptr_t>(g->D3) % 32 == 0;
+        }
+        return launch<FMODE_WGRAD>(m, p, g->G * ((g->M + TILE_M - 1) / TILE_M) * ((g->N + BN - 1) / BN) * p.products, stream);
     }
     MOKB_REQUIRE(g->K > 0 && g->K % 128 == 0 && g->N > 0 && g->N % 128 == 0, "grouped_gemm_mxfp8: K and N must be multiples of 128");
     const uint64_t brows = static_cast<uint64_t>(g->G) * g->N;

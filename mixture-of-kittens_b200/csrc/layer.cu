@@ -11,7 +11,7 @@
 //   backward  side stream: scaled dispatch of d_y, likewise
 //             caller     : prologue | shared backward (6 launches) | d_hidden = d_y * W_down (one launch, window by window)
 //                          | SwiGLU backward | d_x = d_gate * W_gate + d_up * W_up, whose epilogue stores every row and its
-//                            router-weight gradient into the home rank's buffers | three weight gradients
+//                            router-weight gradient into the home rank's buffers | three weight gradients in one launch
 //
 // The counters are the reference's (csrc/megakernel/utils.cuh:1-13, types.cuh:126-130): global-memory words added to
 // with release semantics by whoever produced some rows and polled with acquire loads by whoever consumes them.  Who may
@@ -52,6 +52,23 @@ int get_async(Async** out) {
     }
     *out = &a;
     return MOKB_OK;
+}
+
+int weight_gradients(const void* d_y, const void* hidden, const void* d_gate, const void* d_up, const void* x, void* d_w_down, void* d_w_gate,
+                     void* d_w_up, int H, int I, int G, int first, int rows, const int32_t* offs, const int32_t* k_end, int accumulate,
+                     int32_t* status, cudaStream_t stream) {
+    mokb_gemm_args w = gemm_base(status);
+    w.mode = 3; w.row_begin = first; w.rows_static = rows; w.G = G; w.group_offsets = offs; w.group_k_end = k_end; w.accumulate = accumulate;
+    w.A = d_y; w.lda = w.M = H; w.B = hidden; w.ldb = w.ldd = w.N = I; w.D = d_w_down;
+    if (gemm_uses_pairs()) {
+        w.A2 = d_gate; w.B3 = d_up; w.B2 = x; w.D2 = d_w_gate; w.D3 = d_w_up;
+        return mokb_grouped_gemm_bf16(&w, stream);
+    }
+    MOKB_TRY(mokb_grouped_gemm_bf16(&w, stream));
+    w.A = d_gate; w.lda = w.M = I; w.B = x; w.ldb = w.ldd = w.N = H; w.D = d_w_gate;
+    MOKB_TRY(mokb_grouped_gemm_bf16(&w, stream));
+    w.A = d_up; w.D = d_w_up;
+    return mokb_grouped_gemm_bf16(&w, stream);
 }
 
 bool overlap_enabled() {
@@ -187,16 +204,6 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
     MOKB_TRY(run_prologue(a->tokens_per_expert, a->num_tokens, a->peer_rank, E_l, C, MB, T, s, a->status, stream));
     const void* d_y_local = reinterpret_cast<const void*>(static_cast<uintptr_t>(a->d_y_ptrs_host[a->ep_rank]));
     const void* x_local = reinterpret_cast<const void*>(static_cast<uintptr_t>(a->x_ptrs_host[a->ep_rank]));
-    // A and B as they lie in memory: `rows` rows, the first of which is row `first` in the numbering of `offs`
-    auto wgrad = [&](const void* A, int M, const void* B, int N, void* D, int G, int first, int rows, const int32_t* offs, int accumulate,
-                     const int32_t* k_end = nullptr) -> int {
-        mokb_gemm_args w = gemm_base(a->status);
-        w.mode = 3; w.row_begin = first; w.rows_static = rows; w.G = G; w.M = M; w.N = N; w.group_offsets = offs; w.accumulate = accumulate;
-        w.group_k_end = k_end;       // the padding rows at the end of every expert's segment are zero: not multiplied
-        w.A = A; w.lda = M; w.B = B; w.ldb = N; w.D = D; w.ldd = N;
-        return mokb_grouped_gemm_bf16(&w, stream);
-    };
-
     for (int m = 0; m < n_macro; ++m) {
         const int lo = m * MB, hi = (lo + MB < C) ? lo + MB : C;
         // the saved context and the routed work buffers, addressed by schedule row
@@ -243,9 +250,8 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
             g.A = a->d_gate_shared; g.B = a->w_shared_gate; g.A2 = a->d_up_shared; g.B2 = a->w_shared_up; g.lda = I; g.ldb = H;
             g.D = a->d_x_shared; g.ldd = H;
             MOKB_TRY(mokb_grouped_gemm_bf16(&g, stream));
-            MOKB_TRY(wgrad(d_y_local, H, a->hidden_shared, I, a->d_w_shared_down, 1, 0, T, s.shared_offsets, 0));
-            MOKB_TRY(wgrad(a->d_gate_shared, I, x_local, H, a->d_w_shared_gate, 1, 0, T, s.shared_offsets, 0));
-            MOKB_TRY(wgrad(a->d_up_shared, I, x_local, H, a->d_w_shared_up, 1, 0, T, s.shared_offsets, 0));
+            MOKB_TRY(weight_gradients(d_y_local, a->hidden_shared, a->d_gate_shared, a->d_up_shared, x_local, a->d_w_shared_down, a->d_w_shared_gate,
+                                      a->d_w_shared_up, H, I, 1, 0, T, s.shared_offsets, nullptr, 0, a->status, stream));
         }
 
         // ---- routed experts of this macrobatch
@@ -285,9 +291,9 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
         MOKB_TRY(mokb_grouped_gemm_bf16(&g, stream));
         const int32_t* offs = s.mb_offsets + static_cast<size_t>(m) * (E_l + 1);
         const int32_t* k_end = s.mb_k_end + static_cast<size_t>(m) * (E_l + 1);
-        MOKB_TRY(wgrad(a->d_y_routed, H, a->hidden_routed, I, a->d_w_routed_down, E_l, lo, hi - lo, offs, m > 0, k_end));
-        MOKB_TRY(wgrad(a->d_gate_routed, I, a->x_routed, H, a->d_w_routed_gate, E_l, lo, hi - lo, offs, m > 0, k_end));
-        MOKB_TRY(wgrad(a->d_up_routed, I, a->x_routed, H, a->d_w_routed_up, E_l, lo, hi - lo, offs, m > 0, k_end));
+        // the padding rows at the end of every expert's segment are zero: not multiplied
+        MOKB_TRY(weight_gradients(a->d_y_routed, a->hidden_routed, a->d_gate_routed, a->d_up_routed, a->x_routed, a->d_w_routed_down,
+                                  a->d_w_routed_gate, a->d_w_routed_up, H, I, E_l, lo, hi - lo, offs, k_end, m > 0, a->status, stream));
     }
     return MOKB_OK;
 }

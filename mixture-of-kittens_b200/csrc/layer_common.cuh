@@ -205,6 +205,11 @@ struct Async {
 
 int get_async(Async** out);      // layer.cu
 bool overlap_enabled();          // layer.cu
+// The three weight gradients of G experts over `rows` rows, the first of which is row `first` in the numbering of `offs`
+// (layer.cu): d_w_down [G][H, I] = d_y^T hidden, d_w_gate / d_w_up [G][I, H] = d_gate^T x / d_up^T x.
+int weight_gradients(const void* d_y, const void* hidden, const void* d_gate, const void* d_up, const void* x, void* d_w_down, void* d_w_gate,
+                     void* d_w_up, int H, int I, int G, int first, int rows, const int32_t* offs, const int32_t* k_end, int accumulate,
+                     int32_t* status, cudaStream_t stream);
 
 namespace {
 

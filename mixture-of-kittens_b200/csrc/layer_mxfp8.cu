@@ -280,15 +280,8 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
             g.A = a->d_gate_shared; g.B = a->w_shared_gate; g.A2 = a->d_up_shared; g.B2 = a->w_shared_up; g.lda = I; g.ldb = H;
             g.D = a->d_x_shared; g.ldd = H;
             MOKB_TRY(mokb_grouped_gemm_bf16(&g, stream));
-            auto wgrad_bf16 = [&](const void* A, int M, const void* B, int N, void* D) -> int {
-                mokb_gemm_args w = gemm_base(a->status);
-                w.mode = 3; w.rows_static = T; w.G = 1; w.M = M; w.N = N; w.group_offsets = s.shared_offsets;
-                w.A = A; w.lda = M; w.B = B; w.ldb = N; w.D = D; w.ldd = N;
-                return mokb_grouped_gemm_bf16(&w, stream);
-            };
-            MOKB_TRY(wgrad_bf16(d_y_local, H, a->hidden_shared, I, a->d_w_shared_down));
-            MOKB_TRY(wgrad_bf16(a->d_gate_shared, I, x_local, H, a->d_w_shared_gate));
-            MOKB_TRY(wgrad_bf16(a->d_up_shared, I, x_local, H, a->d_w_shared_up));
+            MOKB_TRY(weight_gradients(d_y_local, a->hidden_shared, a->d_gate_shared, a->d_up_shared, x_local, a->d_w_shared_down, a->d_w_shared_gate,
+                                      a->d_w_shared_up, H, I, 1, 0, T, s.shared_offsets, nullptr, 0, a->status, stream));
         }
 
         // ---- routed experts of this macrobatch (MXFP8)
@@ -319,17 +312,14 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
         MOKB_TRY(mokb_grouped_gemm_mxfp8(&f, stream));
         const int32_t* offs = s.mb_offsets + static_cast<size_t>(m) * (E_l + 1);
         const int32_t* k_end = s.mb_k_end + static_cast<size_t>(m) * (E_l + 1);
-        auto wgrad_fp8 = [&](const void* A, const void* A_sc, int M, const void* B, const void* B_sc, int N, void* D) -> int {
-            mokb_gemm_fp8_args w = fp8_base(a->status);
-            w.mode = 2; w.rows_static = MB; w.t_first = lo; w.G = E_l; w.M = M; w.N = N; w.group_offsets = offs; w.accumulate = m > 0;
-            w.group_k_end = k_end;       // a segment's padding may fill a whole 128-token stage of zeros
-            w.A = A; w.A_sc = A_sc; w.B = B; w.B_sc = B_sc; w.D = D; w.ldd = N;
-            return mokb_grouped_gemm_mxfp8(&w, stream);
-        };
-        // the token-wise tensors are passed as they lie in memory ([., MB], first token column = lo)
-        MOKB_TRY(wgrad_fp8(a->d_gate_fp8_t, a->d_gate_sc_t, I, a->x_fp8_t, a->x_sc_t, H, a->d_w_routed_gate));
-        MOKB_TRY(wgrad_fp8(a->d_up_fp8_t, a->d_up_sc_t, I, a->x_fp8_t, a->x_sc_t, H, a->d_w_routed_up));
-        MOKB_TRY(wgrad_fp8(a->d_y_fp8_t, a->d_y_sc_t, H, a->hidden_fp8_t, a->hidden_sc_t, I, a->d_w_routed_down));
+        // the three weight gradients in one launch; the token-wise tensors are passed as they lie in memory ([., MB], first token
+        // column = lo), and where a segment's padding fills a whole 128-token stage of zeros, that stage is left out
+        f = fp8_base(a->status);
+        f.mode = 2; f.rows_static = MB; f.t_first = lo; f.G = E_l; f.M = H; f.N = I; f.group_offsets = offs; f.group_k_end = k_end; f.accumulate = m > 0;
+        f.A = a->d_y_fp8_t; f.A_sc = a->d_y_sc_t; f.B = a->hidden_fp8_t; f.B_sc = a->hidden_sc_t; f.D = a->d_w_routed_down; f.ldd = I;
+        f.A2 = a->d_gate_fp8_t; f.A2_sc = a->d_gate_sc_t; f.B3 = a->d_up_fp8_t; f.B3_sc = a->d_up_sc_t; f.B2 = a->x_fp8_t; f.B2_sc = a->x_sc_t;
+        f.D2 = a->d_w_routed_gate; f.D3 = a->d_w_routed_up;
+        MOKB_TRY(mokb_grouped_gemm_mxfp8(&f, stream));
     }
     return MOKB_OK;
 }

@@ -92,7 +92,7 @@ class GemmFp8Args(ctypes.Structure):
         + [("B3", c_vp), ("B3_sc", c_vp), ("N2", c_int), ("window_rows", c_int), ("win_ready", c_vp), ("win_ready_target", c_int),
            ("blk_done", c_vp), ("win_done", c_vp), ("push_ptrs_host", c_u64p), ("push_ep_size", c_int), ("push_rank", c_vp),
            ("push_idx", c_vp), ("push_values", c_vp), ("push_value_ptrs_host", c_u64p), ("push_index_limit", c_i64),
-           ("reserve_sms", c_int), ("group_k_end", c_vp)])
+           ("reserve_sms", c_int), ("group_k_end", c_vp), ("D3", c_vp)])
 
 
 def _sig(name, restype, *argtypes):
@@ -524,13 +524,13 @@ def grouped_gemm_mxfp8(mode, A, A_sc, B, B_sc, D, *, rows=None, num_rows=None, g
                        t_first=0, accumulate=False, quantised_outputs=None, t_rows=0, swiglu_limit=None, B3=None, B3_sc=None,
                        N2=0, window_rows=0, win_ready=None, win_ready_target=0, blk_done=None, win_done=None, push_ptrs=None,
                        push_rank=None, push_idx=None, push_values=None, push_value_ptrs=None, reserve_sms=0,
-                       push_index_limit=0, group_k_end=None):
+                       push_index_limit=0, group_k_end=None, D3=None):
     """`quantised_outputs` (modes 3, 4): (gate_q, gate_sc, up_q, up_sc, hid_q, hid_sc, hid_qt, hid_sct); D is unused in
     mode 3 and the down projection's output [rows, N2] in mode 4 (B3, B3_sc: its weights)."""
     g = GemmFp8Args()
     g.B3, g.B3_sc, g.N2 = _p(B3), _p(B3_sc), N2
     g.reserve_sms = reserve_sms
-    g.group_k_end = _p(group_k_end)
+    g.group_k_end, g.D3 = _p(group_k_end), _p(D3)
     g.window_rows, g.win_ready, g.win_ready_target = window_rows, _p(win_ready), win_ready_target
     g.blk_done, g.win_done = _p(blk_done), _p(win_done)
     keep = []

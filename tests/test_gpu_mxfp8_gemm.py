@@ -147,6 +147,26 @@ def test_mxfp8_gemm_wgrad(cols_per_group, M, N):
         assert_close(f"wgrad {gi}", ref, D[gi], (GEMM_TOL[0] * 8, GEMM_TOL[1]))
 
 
+@pytest.mark.parametrize("cols_per_group,M,N", [([512, 0, 256], 256, 384), ([256, 768], 640, 128)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_mxfp8_three_weight_gradients_in_one_launch_equal_three_launches(cols_per_group, M, N, accumulate):
+    from mok import _C
+    offs, gob, cols = groups(cols_per_group)
+    G_ = len(cols_per_group)
+    g = torch.Generator().manual_seed(36)
+    (A, As, _), (B, Bs, _), (A2, A2s, _), (B2, B2s, _), (B3, B3s, _) = (
+        quant(torch.randn(n, cols, generator=g).to(torch.bfloat16)) for n in (M, N, N, M, N))
+    start = [torch.randn(G_, *s, generator=g).to(torch.bfloat16).cuda() for s in ((M, N), (N, M), (N, M))]
+    want, got = [t.clone() for t in start], [t.clone() for t in start]
+    for (a, a_s, b, b_s, m, n), d in zip(((A, As, B, Bs, M, N), (A2, A2s, B2, B2s, N, M), (B3, B3s, B2, B2s, N, M)), want):
+        _C.grouped_gemm_mxfp8(2, a, a_s, b, b_s, d, group_offsets=offs, G=G_, M=m, N=n, accumulate=accumulate)
+    _C.grouped_gemm_mxfp8(2, A, As, B, Bs, got[0], group_offsets=offs, G=G_, M=M, N=N, accumulate=accumulate, A2=A2, A2_sc=A2s, B2=B2, B2_sc=B2s,
+                          B3=B3, B3_sc=B3s, D2=got[1], D3=got[2])
+    torch.cuda.synchronize()
+    assert _C.check_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
 def test_mxfp8_gemm_wgrad_leaves_out_the_padding_tokens_it_is_told_about():
     """group_k_end: tokens of a group from there on are zero in both operands.  The kernel stops at the next multiple of
     128 tokens, so whatever lies beyond that -- E4M3 NaN here -- must not reach the result."""

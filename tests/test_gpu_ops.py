@@ -377,3 +377,22 @@ def test_gemm_wgrad_leaves_out_the_padding_rows_it_is_told_about(mods):
             continue
         ref = (A[s:e].float().T @ B[s:e].float()).to(torch.bfloat16)
         assert_close(f"wgrad group {i}", ref, D[i], (GEMM_TOL[0] * 8, GEMM_TOL[1]))
+
+
+@pytest.mark.parametrize("rows_per_group,M,N", [([512, 0, 256], 256, 384), ([256], 512, 128), ([768, 256], 768, 640)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_gemm_three_weight_gradients_in_one_launch_equal_three_launches(mods, rows_per_group, M, N, accumulate):
+    _C, ops = mods
+    offs, gob, rows = _groups(rows_per_group)
+    G_ = len(rows_per_group)
+    g = torch.Generator().manual_seed(19)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).cuda()
+    A, B, A2, B2, B3 = rnd(rows, M), rnd(rows, N), rnd(rows, N), rnd(rows, M), rnd(rows, N)
+    start = (rnd(G_, M, N), rnd(G_, N, M), rnd(G_, N, M))
+    want, got = [t.clone() for t in start], [t.clone() for t in start]
+    for (a, b, m, n), d in zip(((A, B, M, N), (A2, B2, N, M), (B3, B2, N, M)), want):
+        _C.grouped_gemm(3, a, b, d, group_offsets=offs, G=G_, M=m, N=n, accumulate=accumulate)
+    _C.grouped_gemm(3, A, B, got[0], group_offsets=offs, G=G_, M=M, N=N, accumulate=accumulate, A2=A2, B2=B2, B3=B3, D2=got[1], D3=got[2])
+    torch.cuda.synchronize()
+    assert _C.check_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
