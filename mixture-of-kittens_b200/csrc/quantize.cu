@@ -268,12 +268,12 @@ __global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
                     g = fminf(g, c.limit);
                     u = fminf(fmaxf(u, -c.limit), c.limit);
                 }
-                const float sig = 1.0f / (1.0f + __expf(-g));
+                const float sig = __fdividef(1.0f, 1.0f + __expf(-g));
                 const float silu = g * sig;
                 const float dsilu = (1.0f - silu) * sig + silu;
                 dg[j] = g_ok ? dsilu * u * dhv[j] : 0.0f;
                 du[j] = u_ok ? silu * dhv[j] : 0.0f;
-                partial += dhv[j] * inv_w * (silu * u);
+                partial += dhv[j] * (silu * u);
             }
             wg[i] = pack2(dg[0], dg[1]);
             wu[i] = pack2(du[0], du[1]);
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
         if (partials) {
 #pragma unroll
             for (int d = 4; d >= 1; d >>= 1) partial += __shfl_xor_sync(0xffffffffu, partial, d);
-            if (seg == 0) partials[row * (I >> 7) + blockIdx.x] = partial;
+            if (seg == 0) partials[row * (I >> 7) + blockIdx.x] = partial * inv_w;
         }
     }
     __syncthreads();
