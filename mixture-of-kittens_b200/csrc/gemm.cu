@@ -5,7 +5,7 @@
 //
 //   warp 0      TMA producer   (one lane)  : global -> smem ring
 //   warp 1      MMA issuer     (one lane)  : 4 x tcgen05.mma (K = 16 each) per 64-wide K stage
-//   warps 2..5  epilogue                   : TMEM -> registers -> bf16 -> global
+//   warps 2..   epilogue (4; 8 for weight gradients) : TMEM -> registers -> bf16 -> global
 //
 // Two tile shapes share the code (template parameter NCTA):
 //   NCTA = 2  a pair of CTAs on neighbouring SMs (cluster of 2, tcgen05 cta_group::2) computes a
@@ -51,7 +51,10 @@ namespace {
 constexpr int BN = 256, BK = 64;
 constexpr int A_BYTES = 128 * BK * 2;           // 16 KB: 128 rows (or 2 x 64 columns) of A per CTA
 constexpr int CHUNK_BYTES = 64 * BK * 2;        // one 64-wide MN-major chunk: 8 KB
-constexpr int NUM_THREADS = 192;
+// Epilogue warps.  Weight gradients take two per quarter of tensor memory: an expert's rows are the contraction there, and
+// with few of them (384: six stages) a tile's epilogue is longer than its main loop.  The other modes have one per quarter and
+// leave the registers to the kernels that run beside them.
+template <int MODE> constexpr int kEpilogueWarps = MODE == 3 ? 8 : 4;
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_ROWS = 1024;                // rows per raster super-group
 
@@ -333,7 +336,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(tfull_bar(a), 1);
-            mbar_init(tempty_bar(a), 4 * NCTA);   // leader's: one arrival per epilogue warp of the pair
+            mbar_init(tempty_bar(a), kEpilogueWarps<MODE> * NCTA);   // leader's: one arrival per epilogue warp of the pair
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -495,7 +498,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
         }
     } else {
-        // ------------------------------------------------------------ epilogue (warps 2..5 of every CTA)
+        // ------------------------------------------------------------ epilogue (warps 2.. of every CTA)
         const int quarter = warp & 3;                   // TMEM lanes [32q, 32q+32) belong to warps with id % 4 == q
         const int row_in_cta = quarter * 32 + lane;
         int local = 0;
@@ -552,23 +555,89 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         store_row32(p.D3 + off + c * 32, hw, p.wide_stores);
                     }
                 }
+            } else if (MODE == MODE_WGRAD) {
+                // this warp: 32 rows x 128 columns of this product's [M, N]
+                const int half = (warp - 2) >> 2;
+                const int rows_all = ti.phase ? p.N : p.M, cols_all = ti.phase ? p.M : p.N;
+                const int row0 = ti.m_blk * G::TILE_M + row_in_tile - lane, col0 = ti.n_blk * BN + half * 128;
+                const int ld_out = ti.phase ? p.M : p.ldd;
+                const int live_rows = min(32, rows_all - row0), nchunks = min(4, (cols_all - col0 + 31) / 32);
+                __nv_bfloat16* const warp_dst = (ti.phase == 0 ? p.D : ti.phase == 1 ? p.D2 : p.D3) +
+                                                (static_cast<size_t>(ti.group) * rows_all + row0) * ld_out + col0;
+                const uint32_t t_cols = t_addr + half * 128;
+                if (nchunks <= 0 || (empty_k && p.accumulate)) {
+                    // no columns of the matrix, or nothing to add: the stored gradient stays
+                } else if (empty_k || p.accumulate || !p.line_stores) {
+                    // register path: a lane stores its own row, 32 bytes at a time
+                    __nv_bfloat16* const dst = warp_dst + static_cast<size_t>(lane) * ld_out;
+#pragma unroll 1
+                    for (int c = 0; c < nchunks; ++c) {
+                        uint32_t r[32];
+                        __syncwarp();
+                        tmem_ld_32x32(t_cols + c * 32, r);         // (whole warp, also for unstored rows)
+                        tmem_ld_wait_for(r);
+                        if (lane >= live_rows) continue;
+                        if (empty_k) {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) r[i] = 0u;
+                        }
+                        if (p.accumulate) {
+                            const uint4* old = reinterpret_cast<const uint4*>(dst + c * 32);
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                const uint4 o = old[q];
+                                const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const float2 f = unpack_bf16(ow[j]);
+                                    r[8 * q + 2 * j] = __float_as_uint(__uint_as_float(r[8 * q + 2 * j]) + f.x);
+                                    r[8 * q + 2 * j + 1] = __float_as_uint(__uint_as_float(r[8 * q + 2 * j + 1]) + f.y);
+                                }
+                            }
+                        }
+                        store_row32(dst + c * 32, r, p.wide_stores);
+                    }
+                    __syncwarp();
+                } else {
+                    // line path (see below) through 2 KB per warp, 32 columns at a time: four lanes store 64 bytes of a row.
+                    // The tensor-memory load of the next 32 columns is in flight meanwhile.
+                    const uint32_t stage = bars + 256u + static_cast<uint32_t>(warp - 2) * 2048u;
+                    const int sub = lane >> 2, unit = lane & 3;
+                    uint32_t r[32];
+                    tmem_ld_32x32(t_cols, r);
+#pragma unroll 1
+                    for (int c = 0; c < nchunks; ++c) {
+                        uint32_t w[16];
+                        tmem_ld_wait_for(r);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) w[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                        __syncwarp();             // the previous columns have been read out of the buffer
+                        if (c + 1 < nchunks) tmem_ld_32x32(t_cols + (c + 1) * 32, r);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)      // row `lane`, 16-byte unit u at u ^ ((lane >> 1) & 3): conflict-free both ways
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + lane * 64u + static_cast<uint32_t>((u ^ ((lane >> 1) & 3)) << 4)),
+                                         "r"(w[4 * u]), "r"(w[4 * u + 1]), "r"(w[4 * u + 2]), "r"(w[4 * u + 3]) : "memory");
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int rr = 8 * i + sub;
+                            uint32_t v0, v1, v2, v3;
+                            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
+                                         : "r"(stage + rr * 64u + static_cast<uint32_t>((unit ^ ((rr >> 1) & 3)) << 4)) : "memory");
+                            if (rr < live_rows) st_global_v4(warp_dst + static_cast<size_t>(rr) * ld_out + c * 32 + unit * 8, v0, v1, v2, v3);
+                        }
+                    }
+                }
             } else {
                 const int tile_row = ti.m_blk * G::TILE_M + row_in_tile;
                 bool row_ok = true;
-                size_t row;
-                const int wg_m = ti.phase ? p.N : p.M, wg_n = ti.phase ? p.M : p.N;      // MODE_WGRAD: this product's [M, N]
-                if (MODE == MODE_WGRAD) {
-                    row_ok = tile_row < wg_m;
-                    row = static_cast<size_t>(ti.group) * wg_m + tile_row;
-                } else {
-                    row = static_cast<size_t>(tile_row);
-                }
-                __nv_bfloat16* const base = MODE == MODE_FWD ? p.D4 : MODE == MODE_WGRAD && ti.phase ? (ti.phase == 1 ? p.D2 : p.D3) : p.D;
-                const size_t ld_out = MODE == MODE_FWD ? p.ldd4 : MODE == MODE_WGRAD && ti.phase ? p.M : p.ldd;
+                const size_t row = static_cast<size_t>(tile_row);
+                __nv_bfloat16* const base = MODE == MODE_FWD ? p.D4 : p.D;
+                const size_t ld_out = MODE == MODE_FWD ? p.ldd4 : p.ldd;
                 __nv_bfloat16* dst = base + row * ld_out + static_cast<size_t>(ti.n_blk) * BN;
                 if (base == nullptr) row_ok = false;          // pushed only
                 __nv_bfloat16* pdst = nullptr;                // this row's place in its home rank's buffer
-                if ((MODE == MODE_NT || MODE == MODE_NN || MODE == MODE_FWD) && p.push) {
+                if (p.push) {
                     const int pr = p.push_rank[tile_row];
                     if (pr >= 0 && pr < p.push_ranks &&
                         index_ok(IndexGuard{p.push_limit, p.status}, p.push_idx[tile_row], kBadIndexGemmPush, tile_row)) {
@@ -577,37 +646,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         if (p.push_values && ti.n_blk == 0) static_cast<float*>(p.push_val.p[pr])[slot] = p.push_values[tile_row];
                     }
                 }
-                const int cols_left = (MODE == MODE_FWD ? p.N2 : MODE == MODE_WGRAD ? wg_n : p.N) - ti.n_blk * BN;
+                const int cols_left = (MODE == MODE_FWD ? p.N2 : p.N) - ti.n_blk * BN;
                 const int nchunks = min(BN / 32, (cols_left + 31) / 32);
-                // one 32-column chunk from registers: (optionally add the stored gradient,) round to bf16, store locally
-                // and / or at home
+                // one 32-column chunk from registers: round to bf16, store locally and / or at home
                 auto put = [&](uint32_t (&r)[32], int c) {
-                    if (MODE == MODE_WGRAD && p.accumulate && row_ok) {
-                        const uint4* old = reinterpret_cast<const uint4*>(dst + c * 32);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const uint4 o = old[q];
-                            const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const float2 f = unpack_bf16(ow[j]);
-                                r[8 * q + 2 * j] = __float_as_uint(__uint_as_float(r[8 * q + 2 * j]) + f.x);
-                                r[8 * q + 2 * j + 1] = __float_as_uint(__uint_as_float(r[8 * q + 2 * j + 1]) + f.y);
-                            }
-                        }
-                    }
                     if (row_ok) store_row32(dst + c * 32, r, p.wide_stores);
                     if (pdst) store_row32(pdst + c * 32, r, p.push_wide);
                 };
-                if (empty_k) {
-                    if (!(MODE == MODE_WGRAD && p.accumulate)) {      // accumulate: nothing to add, leave the stored gradient
-                        uint32_t z[32];
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) z[i] = 0u;
-#pragma unroll 1
-                        for (int c = 0; c < nchunks; ++c) put(z, c);
-                    }
-                } else if ((MODE == MODE_WGRAD && p.accumulate) || (nchunks & 1) || !p.line_stores) {
+                if ((nchunks & 1) || !p.line_stores) {
                     // register path: a lane stores its own row, 32 bytes at a time.  Two register sets: the tensor-memory
                     // load of the next chunk is in flight while this one is stored (whole warp, also for unstored rows)
                     uint32_t ra[32], rb[32];
@@ -634,7 +680,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     const int sub = lane >> 3, unit = lane & 7;
                     // lane 0's row of the local output (rows of a warp are consecutive) and this lane's own row at home
                     __nv_bfloat16* const warp_dst = base ? dst - static_cast<size_t>(lane) * ld_out : nullptr;
-                    const int warp_row0 = tile_row - lane;
                     const unsigned long long own_home = reinterpret_cast<unsigned long long>(pdst);
                     const int npairs = nchunks >> 1;
 #pragma unroll 1
@@ -665,9 +710,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                             uint32_t v0, v1, v2, v3;
                             asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
                                          : "r"(stage + rr * 128u + static_cast<uint32_t>((unit ^ (rr & 7)) << 4)) : "memory");
-                            if (warp_dst && (MODE != MODE_WGRAD || warp_row0 + rr < wg_m))
-                                st_global_v4(warp_dst + static_cast<size_t>(rr) * ld_out + col, v0, v1, v2, v3);
-                            if ((MODE == MODE_NT || MODE == MODE_NN || MODE == MODE_FWD) && p.push) {
+                            if (warp_dst) st_global_v4(warp_dst + static_cast<size_t>(rr) * ld_out + col, v0, v1, v2, v3);
+                            if (p.push) {
                                 __nv_bfloat16* home = reinterpret_cast<__nv_bfloat16*>(__shfl_sync(0xffffffffu, own_home, rr));
                                 if (home) st_global_v4(home + col, v0, v1, v2, v3);
                             }
@@ -719,7 +763,7 @@ int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2, co
     if (units < 1) return MOKB_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(units * NCTA));
-    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.blockDim = dim3(64 + 32 * kEpilogueWarps<MODE>);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
