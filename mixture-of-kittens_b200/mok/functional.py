@@ -340,6 +340,17 @@ def _stage(buffer: torch.Tensor, value: torch.Tensor) -> None:
     buffer.copy_(value)
 
 
+def _input(ws: MoKWorkspace, buffer: torch.Tensor, ptrs: list[int], value: torch.Tensor) -> tuple[torch.Tensor, list[int]]:
+    """The tensor the kernels read `value` from, and its address on every rank: the symmetric `buffer` after staging, or,
+    where no other rank reads it, `value` itself (on one rank the copy of 16384 x 7168 activations takes 75 us and three of
+    them a hundredth of a training step; of 1024 x 1024, 2 us and 6 us of host time each).  The kernels read 32 bytes at a
+    time, so a value that is not aligned to that is staged; so is whatever the operators do not run on directly."""
+    if ws.ep_size == 1 and ops.runs_directly(value) and value.data_ptr() % 32 == 0:
+        return value, [value.data_ptr()]
+    _stage(buffer, value)
+    return buffer, ptrs
+
+
 def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x: torch.Tensor,
             router_weights: torch.Tensor, shared_gate_weights: torch.Tensor, shared_up_weights: torch.Tensor,
             shared_down_weights: torch.Tensor, routed_gate_weights, routed_up_weights, routed_down_weights,
@@ -348,8 +359,8 @@ def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x
     [E_l, I, H] / [E_l, H, I], or (fp8, scales) pairs for MXFP8."""
     validate_inputs(config, workspace, schedule, x, router_weights)
     ws = workspace
-    _stage(ws.x_buffer, x)
-    _stage(ws.router_weight_buffer, router_weights)
+    x_in, x_ptrs = _input(ws, ws.x_buffer, ws.x_buffer_ptrs, x)
+    weights_in, _ = _input(ws, ws.router_weight_buffer, ws.router_weight_buffer_ptrs, router_weights)
     _barrier(ws)
     if _is_mxfp8(routed_gate_weights):
         from . import ops_mxfp8
@@ -357,7 +368,7 @@ def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x
         (x_fp8_t, x_sc_t, gate_shared, gate_fp8, gate_sc, up_shared, up_fp8, up_sc, hidden_shared, hidden_fp8_t,
          hidden_sc_t, y_shared, _y_routed) = ops.call(
             ops_mxfp8.dispatch_mlp_swiglu_combine_fwd_mxfp8,
-            ws.x_buffer, ws.x_buffer_ptrs, ws.combine_buffer, ws.combine_buffer_ptrs,
+            x_in, x_ptrs, ws.combine_buffer, ws.combine_buffer_ptrs,
             shared_gate_weights, gq, gs, shared_up_weights, uq, us, shared_down_weights, dq, ds,
             schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert,
             ws.topk, swiglu_limit, config.fwd_num_comm_sms, config.macrobatch_size, config.minibatch_size)
@@ -368,7 +379,7 @@ def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x
         (x_routed, gate_shared, gate_routed, up_shared, up_routed, hidden_shared, hidden_routed, y_shared,
          _y_routed) = ops.call(
             ops.dispatch_mlp_swiglu_combine_fwd_bf16,
-            ws.x_buffer, ws.x_buffer_ptrs, ws.combine_buffer, ws.combine_buffer_ptrs,
+            x_in, x_ptrs, ws.combine_buffer, ws.combine_buffer_ptrs,
             shared_gate_weights, routed_gate_weights, shared_up_weights, routed_up_weights,
             shared_down_weights, routed_down_weights,
             schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert,
@@ -377,7 +388,7 @@ def forward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, x
                                 up_shared=up_shared, up_routed=up_routed, hidden_shared=hidden_shared,
                                 hidden_routed=hidden_routed)
     _barrier(ws)
-    output = ops.call(ops.fwd_epilogue, y_shared, ws.combine_buffer, ws.router_weight_buffer)
+    output = ops.call(ops.fwd_epilogue, y_shared, ws.combine_buffer, weights_in)
     return output, ctx
 
 
@@ -392,7 +403,7 @@ def recompute_forward_context(config: MoKConfig, workspace: MoKWorkspace, schedu
     if _is_mxfp8(routed_gate_weights) and (len(routed_gate_weights) != 2 or len(routed_up_weights) != 2):
         raise ValueError("MXFP8 routed gate and up weights must be data/scale pairs")
     ws = workspace
-    _stage(ws.x_buffer, x)
+    x_in, x_ptrs = _input(ws, ws.x_buffer, ws.x_buffer_ptrs, x)
     _barrier(ws)
     if _is_mxfp8(routed_gate_weights):
         from . import ops_mxfp8
@@ -400,7 +411,7 @@ def recompute_forward_context(config: MoKConfig, workspace: MoKWorkspace, schedu
         (x_fp8_t, x_sc_t, gate_shared, gate_fp8, gate_sc, up_shared, up_fp8, up_sc, hidden_shared, hidden_fp8_t,
          hidden_sc_t) = ops.call(
             ops_mxfp8.recompute_forward_context_mxfp8,
-            ws.x_buffer, ws.x_buffer_ptrs, shared_gate_weights, gq, gs, shared_up_weights, uq, us,
+            x_in, x_ptrs, shared_gate_weights, gq, gs, shared_up_weights, uq, us,
             schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert,
             ws.topk, swiglu_limit, config.fwd_num_comm_sms, config.macrobatch_size, config.minibatch_size)
         ctx = MoKForwardContext(x_routed=(x_fp8_t, x_sc_t), gate_shared=gate_shared, gate_routed=(gate_fp8, gate_sc),
@@ -410,7 +421,7 @@ def recompute_forward_context(config: MoKConfig, workspace: MoKWorkspace, schedu
         (x_routed, gate_shared, gate_routed, up_shared, up_routed, hidden_shared,
          hidden_routed) = ops.call(
             ops.recompute_forward_context_bf16,
-            ws.x_buffer, ws.x_buffer_ptrs, shared_gate_weights, routed_gate_weights, shared_up_weights,
+            x_in, x_ptrs, shared_gate_weights, routed_gate_weights, shared_up_weights,
             routed_up_weights, schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens,
             schedule.tokens_per_expert, ws.topk, swiglu_limit, config.fwd_num_comm_sms, config.macrobatch_size,
             config.minibatch_size)
@@ -432,9 +443,9 @@ def backward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, 
     if not isinstance(forward_context, MoKForwardContext):
         raise TypeError("forward_context must be a MoKForwardContext")
     ws = workspace
-    _stage(ws.d_y_buffer, grad_output)
-    _stage(ws.x_buffer, x)
-    _stage(ws.router_weight_buffer, router_weights)
+    d_y_in, d_y_ptrs = _input(ws, ws.d_y_buffer, ws.d_y_buffer_ptrs, grad_output)
+    x_in, x_ptrs = _input(ws, ws.x_buffer, ws.x_buffer_ptrs, x)
+    weights_in, weights_ptrs = _input(ws, ws.router_weight_buffer, ws.router_weight_buffer_ptrs, router_weights)
     _barrier(ws)
     ctx = forward_context
     if _is_mxfp8(routed_gate_weights):
@@ -444,13 +455,13 @@ def backward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, 
         dtq, dts = routed_down_weights
         outs = ops.call(
             ops_mxfp8.dispatch_mlp_swiglu_combine_bwd_mxfp8,
-            ws.d_y_buffer, ws.d_y_buffer_ptrs, ws.d_x_routed_buffer, ws.d_x_routed_buffer_ptrs,
-            ws.router_weight_buffer, ws.router_weight_buffer_ptrs, ws.d_router_weight_buffer,
+            d_y_in, d_y_ptrs, ws.d_x_routed_buffer, ws.d_x_routed_buffer_ptrs,
+            weights_in, weights_ptrs, ws.d_router_weight_buffer,
             ws.d_router_weight_buffer_ptrs,
             shared_gate_weights, gtq, gts, shared_up_weights, utq, uts, shared_down_weights, dtq, dts,
             ctx.x_routed[0], ctx.x_routed[1], ctx.gate_shared, ctx.gate_routed[0], ctx.gate_routed[1],
             ctx.up_shared, ctx.up_routed[0], ctx.up_routed[1], ctx.hidden_shared, ctx.hidden_routed[0],
-            ctx.hidden_routed[1], ws.x_buffer, ws.x_buffer_ptrs, gq, gs, uq, us,
+            ctx.hidden_routed[1], x_in, x_ptrs, gq, gs, uq, us,
             schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert,
             ws.topk, swiglu_limit, config.bwd_num_comm_sms, config.macrobatch_size, config.minibatch_size)
         d_x_shared = outs[0]
@@ -458,13 +469,13 @@ def backward(config: MoKConfig, workspace: MoKWorkspace, schedule: MoKSchedule, 
     else:
         outs = ops.call(
             ops.dispatch_mlp_swiglu_combine_bwd_bf16,
-            ws.d_y_buffer, ws.d_y_buffer_ptrs, ws.d_x_routed_buffer, ws.d_x_routed_buffer_ptrs,
-            ws.router_weight_buffer, ws.router_weight_buffer_ptrs, ws.d_router_weight_buffer,
+            d_y_in, d_y_ptrs, ws.d_x_routed_buffer, ws.d_x_routed_buffer_ptrs,
+            weights_in, weights_ptrs, ws.d_router_weight_buffer,
             ws.d_router_weight_buffer_ptrs,
             shared_gate_weights, routed_gate_weights, shared_up_weights, routed_up_weights,
             shared_down_weights, routed_down_weights,
             ctx.x_routed, ctx.gate_shared, ctx.gate_routed, ctx.up_shared, ctx.up_routed, ctx.hidden_shared,
-            ctx.hidden_routed, ws.x_buffer, ws.x_buffer_ptrs,
+            ctx.hidden_routed, x_in, x_ptrs,
             schedule.peer_rank, schedule.peer_token_idx, schedule.num_tokens, schedule.tokens_per_expert,
             ws.topk, swiglu_limit, config.bwd_num_comm_sms, config.macrobatch_size, config.minibatch_size)
         d_x_shared = outs[0]

@@ -53,6 +53,11 @@ def _plain_eager(args) -> bool:
     return True
 
 
+def runs_directly(value: torch.Tensor) -> bool:
+    """Whether `call` would run an operator's body on `value` itself: a plain tensor in plain eager mode."""
+    return _plain_eager((value,))
+
+
 def call(op, *args):
     """How `mok.functional` invokes an operator.  Under `torch.compile`, a dispatch or function mode (FakeTensorMode,
     make_fx, ...), a functorch transform, or with tensor subclasses / tensors that require grad, this is `op(*args)`.
