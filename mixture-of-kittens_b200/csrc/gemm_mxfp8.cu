@@ -51,7 +51,7 @@ constexpr int TMEM_COLS = 512;
 constexpr int SF_COL0 = 256;                       // scale columns start after the accumulator
 constexpr int SF_SET_COLS = 16;                    // SFA 4 + SFB 8, padded
 constexpr int GROUP_M = 4;
-// + one 2 KB transposition buffer per epilogue warp (32 rows x 64 bytes) for rows that are pushed to a peer
+// + one 2 KB transposition buffer per epilogue warp (32 rows x 64 bytes) for rows that are pushed to a peer and for the token-wise form of hidden
 constexpr size_t SMEM_BYTES = static_cast<size_t>(STAGES) * (DATA_BYTES + SF_BYTES) + 1024 + 256 + 8 * 2048;
 
 enum { FMODE_NT = 0, FMODE_DUALB = 1, FMODE_WGRAD = 2, FMODE_GATEUP_QUANT = 3, FMODE_FWD = 4 };
@@ -76,7 +76,7 @@ struct FParams {
     int k_tile_origin;               // FMODE_WGRAD: the operands' first token column, in 128-token tiles, in group_offsets' row space
     // FMODE_GATEUP_QUANT outputs: E4M3 [rows, N] + packed scales for gate, up, hidden; hidden also as [N, t_rows]
     uint8_t *gate_q, *gate_sc, *up_q, *up_sc, *hid_q, *hid_sc, *hid_qt, *hid_sct;
-    int t_rows;
+    int t_rows, aligned_t;           // aligned_t: hid_qt is 32-byte aligned
     int has_limit;
     float limit;
     // counters (row-tiled modes; see gemm.cu) and the down projection of FMODE_FWD
@@ -228,6 +228,65 @@ __device__ __forceinline__ void quantize_row_blocks(const uint32_t (&w)[32], uin
         st_global_32B(q + row * N + col0 + b * 32, out);
         sc[scale_offset(row, (col0 >> 5) + b, N >> 7)] = static_cast<uint8_t>(byte);
     }
+}
+
+// Token-wise quantisation of 32 rows x 64 columns held one row per lane (w[j]: columns 2 j, 2 j + 1): lane l ends up with the
+// 32 bytes of columns 2 l and 2 l + 1, to be stored at `dst` and `dst` + t_rows, and with their scale bytes in w[0].
+// The 64 block maxima over the lanes take 31 shuffles (half of the words change lanes at each step, where a full reduction of
+// every word takes 160), every lane works out the two scales of its own columns, and the bytes change lanes through a 2 KB
+// buffer instead of being stored one by one.
+__device__ __forceinline__ void store_token_blocks(uint32_t (&w)[32], uint32_t stage, uint8_t* dst, int64_t t_rows, int aligned) {
+    const int lane = threadIdx.x & 31;
+    uint32_t m[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const bool upper = (lane & 16) != 0;
+        const uint32_t give = upper ? w[i] : w[i + 16], keep = upper ? w[i + 16] : w[i];
+        m[i] = absmax2(keep & 0x7fff7fffu, __shfl_xor_sync(0xffffffffu, give, 16));
+    }
+#pragma unroll
+    for (int half = 8; half >= 1; half >>= 1) {
+        const bool upper = (lane & half) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const uint32_t give = upper ? m[i] : m[i + half], keep = upper ? m[i + half] : m[i];
+            m[i] = absmax2(keep, __shfl_xor_sync(0xffffffffu, give, half));
+        }
+    }
+    float inv_a, inv_b;
+    const uint32_t byte_a = scale_byte(bf16_lo(m[0]), &inv_a);
+    const uint32_t byte_b = scale_byte(bf16_hi(m[0]), &inv_b);
+    __syncwarp();             // the buffer's previous contents have been read
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {       // row j of the buffer: column pair j, two bytes per token; 16-byte unit u at u ^ ((j >> 1) & 3)
+        const float fa = __shfl_sync(0xffffffffu, inv_a, j), fb = __shfl_sync(0xffffffffu, inv_b, j);
+        uint16_t pair;
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(pair) : "f"(bf16_lo(w[j]) * fa), "f"(bf16_hi(w[j]) * fb));
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(stage + j * 64u + static_cast<uint32_t>((((lane >> 3) ^ ((j >> 1) & 3)) << 4) + (lane & 7) * 2)), "h"(pair) : "memory");
+    }
+    __syncwarp();
+    uint32_t a[8], b[8];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {        // eight tokens: bytes a b a b ..
+        uint32_t v0, v1, v2, v3;
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
+                     : "r"(stage + lane * 64u + static_cast<uint32_t>((u ^ ((lane >> 1) & 3)) << 4)) : "memory");
+        a[2 * u] = __byte_perm(v0, v1, 0x6420);
+        a[2 * u + 1] = __byte_perm(v2, v3, 0x6420);
+        b[2 * u] = __byte_perm(v0, v1, 0x7531);
+        b[2 * u + 1] = __byte_perm(v2, v3, 0x7531);
+    }
+    if (aligned) {
+        st_global_32B(dst, a);
+        st_global_32B(dst + t_rows, b);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            dst[i] = static_cast<uint8_t>(a[i >> 2] >> (8 * (i & 3)));
+            dst[t_rows + i] = static_cast<uint8_t>(b[i >> 2] >> (8 * (i & 3)));
+        }
+    }
+    w[0] = byte_a | (byte_b << 8);
 }
 
 struct Maps {        // by-value kernel argument
@@ -468,26 +527,12 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
                 quantize_row_blocks(hw, p.hid_q, p.hid_sc, row, col0, N);
                 // along tokens: the warp's 32 lanes are one 32-token block of each of its 64 columns
                 const int64_t row_blk0 = static_cast<int64_t>(ti.m_blk) * TILE_M + static_cast<int>(cta) * 128 + quarter * 32;
-                uint32_t my_scales = 0u;                    // lane j keeps the two scale bytes of column pair j
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    uint32_t m = hw[j] & 0x7fff7fffu;
-#pragma unroll
-                    for (int d = 16; d >= 1; d >>= 1) m = absmax2(m, __shfl_xor_sync(0xffffffffu, m, d));
-                    float inv_a, inv_b;
-                    const uint32_t byte_a = scale_byte(bf16_lo(m), &inv_a);
-                    const uint32_t byte_b = scale_byte(bf16_hi(m), &inv_b);
-                    uint16_t pair;
-                    asm volatile("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(pair) : "f"(bf16_lo(hw[j]) * inv_a), "f"(bf16_hi(hw[j]) * inv_b));
-                    const int64_t col = col0 + 2 * j;
-                    p.hid_qt[col * p.t_rows + row] = static_cast<uint8_t>(pair & 0xffu);
-                    p.hid_qt[(col + 1) * p.t_rows + row] = static_cast<uint8_t>(pair >> 8);
-                    if (lane == j) my_scales = byte_a | (byte_b << 8);
-                }
+                store_token_blocks(hw, bars + 256u + static_cast<uint32_t>(warp - 2) * 2048u, p.hid_qt + (col0 + 2 * lane) * p.t_rows + row_blk0,
+                                   p.t_rows, p.aligned_t);
                 {
                     const int64_t col = col0 + 2 * lane;
-                    p.hid_sct[scale_offset(col, row_blk0 >> 5, p.t_rows >> 7)] = static_cast<uint8_t>(my_scales & 0xffu);
-                    p.hid_sct[scale_offset(col + 1, row_blk0 >> 5, p.t_rows >> 7)] = static_cast<uint8_t>(my_scales >> 8);
+                    p.hid_sct[scale_offset(col, row_blk0 >> 5, p.t_rows >> 7)] = static_cast<uint8_t>(hw[0] & 0xffu);
+                    p.hid_sct[scale_offset(col + 1, row_blk0 >> 5, p.t_rows >> 7)] = static_cast<uint8_t>(hw[0] >> 8);
                 }
                 if (MODE == FMODE_FWD) {      // this warp's part of the hidden rows is stored: count it for the down tiles
                     __syncwarp();
@@ -772,6 +817,7 @@ extern "C" int mokb_grouped_gemm_mxfp8(const mokb_gemm_fp8_args* g, void* stream
         p.hid_q = static_cast<uint8_t*>(g->hid_q); p.hid_sc = static_cast<uint8_t*>(g->hid_sc);
         p.hid_qt = static_cast<uint8_t*>(g->hid_qt); p.hid_sct = static_cast<uint8_t*>(g->hid_sct);
         p.t_rows = g->t_rows;
+        p.aligned_t = (reinterpret_cast<uintptr_t>(g->hid_qt) & 31) == 0;
         p.has_limit = g->has_swiglu_limit;
         p.limit = g->swiglu_limit;
         if (g->mode == FMODE_FWD) {
