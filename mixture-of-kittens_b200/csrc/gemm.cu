@@ -329,6 +329,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int tile_id0 = NCTA == 2 ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int tile_stride = NCTA == 2 ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
+    const Sched<MODE, NCTA> sched(p);
+    if (sched.total == 0) return;      // no rows (a macrobatch that stayed empty): both CTAs of a pair leave before the set-up
+
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full_bar(s), 1);        // leader's: one arrive.expect_tx by the leader's producer + all TMA bytes
@@ -369,8 +372,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (NCTA == 2) cluster_sync_all();     // the peer's barriers are initialised before anything signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_slot;
-
-    const Sched<MODE, NCTA> sched(p);
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (both CTAs of a pair)

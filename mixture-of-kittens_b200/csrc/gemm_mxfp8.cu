@@ -319,6 +319,9 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
     const int tile_id0 = static_cast<int>(blockIdx.x >> 1);
     const int tile_stride = static_cast<int>(gridDim.x >> 1);
 
+    const Sched<MODE> sched(p);
+    if (sched.total == 0) return;      // no rows (a macrobatch that stayed empty): both CTAs of a pair leave before the set-up
+
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full_bar(s), 1);
@@ -348,8 +351,6 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ Maps tm, const FParams p) {
     cluster_sync_all();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_slot;
-
-    const Sched<MODE> sched(p);
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (both CTAs)
