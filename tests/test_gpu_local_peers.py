@@ -18,6 +18,26 @@ def make_routes(R, T, K, E_l, seed):
     return torch.topk(logits, K, dim=2).indices.to(torch.int32).numpy()
 
 
+@pytest.mark.parametrize("R,T,K,E_l,multiple", [
+    (1, 512, 3, 8, 4),            # one and a half rows of the 1024-wide order, 128 column blocks
+    (1, 512, 1, 1200, 700),       # many experts: fewer column blocks, most segments empty
+    (3, 768, 5, 40, 24),          # a rank count that does not divide the blocks
+    (2, 1024, 4, 3, 0),           # too small a capacity: nothing but -1
+])
+def test_schedule_at_the_edges_of_its_block_split(R, T, K, E_l, multiple):
+    from mok import _C
+    routes = make_routes(R, T, K, E_l, seed=70 + R)
+    C = T * K * R + 256 * multiple if multiple else 512
+    got = _C.schedule(torch.from_numpy(routes).cuda(), E_l, C, R - 1)
+    if not multiple:
+        assert _C.check_status() != 0
+        assert (got[0] == -1).all() and (got[1] == -1).all()
+        return
+    assert _C.check_status() == 0
+    for a, b in zip(O.schedule(routes, E_l, C, R - 1), got):
+        assert torch.equal(torch.from_numpy(a).reshape(-1), b.cpu().reshape(-1))
+
+
 @pytest.mark.parametrize("R,T,K", [(2, 512, 2), (4, 768, 3), (8, 512, 8)])
 def test_all_gather_top_experts_over_local_peers(R, T, K):
     from mok import _C
