@@ -247,9 +247,12 @@ __device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (
 }
 
 // 32 gate and up columns of this warp's rows from tensor memory (rounded to bf16, as pairs) and hidden = silu(gate) * up of the
-// rounded values, clamped at `limit` (infinity: not).  The quotient is a reciprocal and a product: its two units in the last
-// place of fp32 are below what __expf leaves (error against float64 unchanged to seven digits: the rounding to bf16 is all of
-// it), and the IEEE division's branch kept the 32 columns from overlapping.
+// rounded values, clamped at `limit` (infinity: not).  silu's quotient goes through the approximate reciprocal of a quarter of
+// the denominator (of all of it, it would be zero above 2^126: gates between -88.7 and -87.3).  Of every finite bf16 gate with
+// every mantissa of up, 2 of 8.4 million hidden values are another bf16 number than with the IEEE division: ties of the last
+// rounding to one part in 10^7 (2549 and 2547 differ from the rounded float64 value).  The division's branch keeps the 32
+// columns from overlapping (512 tokens over 64 experts of 5120 x 1408, forward: 778 us, with it 973).
+__device__ __forceinline__ float silu_times(float g, float u) { return __fdividef(0.25f * g, fmaf(0.25f, __expf(-g), 0.25f)) * u; }
 __device__ __forceinline__ void load_32_columns(uint32_t taddr, uint32_t (&w)[16]) {
     uint32_t r[32];
     tmem_ld_32x32(taddr, r);
@@ -270,7 +273,7 @@ __device__ __forceinline__ void swiglu_32_columns(uint32_t t_gate, uint32_t t_up
             uf.x = fminf(fmaxf(uf.x, -limit), limit);
             uf.y = fminf(fmaxf(uf.y, -limit), limit);
         }
-        hw[i] = pack_bf16(__fdividef(gf.x, 1.0f + __expf(-gf.x)) * uf.x, __fdividef(gf.y, 1.0f + __expf(-gf.y)) * uf.y);
+        hw[i] = pack_bf16(silu_times(gf.x, uf.x), silu_times(gf.y, uf.y));
     }
 }
 

@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
                     g = fminf(g, c.limit);
                     u = fminf(fmaxf(u, -c.limit), c.limit);
                 }
-                const float sig = __fdividef(1.0f, 1.0f + __expf(-g));
+                const float sig = 1.0f / (1.0f + __expf(-g));      // (IEEE: __fdividef is zero for gates between -88.7 and -87.3)
                 const float silu = g * sig;
                 const float dsilu = (1.0f - silu) * sig + silu;
                 dg[j] = g_ok ? dsilu * u * dhv[j] : 0.0f;

@@ -1,6 +1,8 @@
 """GPU parity of the MXFP8 layer (routed experts in block-scaled E4M3) through mok.functional at EP = 1:
 against the CPU oracle's MXFP8 dataflow (tight) and against the BF16 result under the reference's
 MXFP8 tolerance (max abs <= 1.0, relative <= 0.1; tests/utils.py:8 of the reference)."""
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -126,3 +128,35 @@ def test_mxfp8_several_macrobatches_with_replay_match_the_single_macrobatch_resu
     # bit-reproducible across runs
     _, outb, _, _, gb, _ = run_mxfp8(ranks[0], 4, MB=MB, mb=mb)
     assert torch.equal(outm, outb) and all(torch.equal(a, b) for a, b in zip(gm, gb))
+
+
+def uniform_mxfp8_backward(T=512, H=256, I=128, *, x, gate, up, w_down, grad_output, router_weight):
+    """The MXFP8 backward of one expert whose saved gate and up, x, down weights, grad_output and router weights are constants
+    (powers of two, or exact in E4M3): d_hidden = router_weight * grad_output * w_down * H exactly.  Returns the gradients by name."""
+    from mok import _C, functional as F, ops
+    full = lambda v, *shape: torch.full(shape, v, dtype=torch.bfloat16, device="cuda")
+    cfg = F.MoKConfig(minibatch_size=256, macrobatch_size=2 * T)
+    ws = F.create_workspace(cfg, init_single_rank_group(), device=torch.device("cuda", 0), num_local_tokens=T, hidden_size=H, topk=1)
+    sched = F.build_schedule(ws, cfg, torch.zeros(T, 1, dtype=torch.int64, device="cuda"), num_local_experts=1)
+    shared = full(0.0, I, H), full(0.0, I, H), full(0.0, H, I)
+    quant = lambda t: ops.mxfp8_quantize(t, True, True)
+    wg, wu, wd = quant(full(0.0, 1, I, H)), quant(full(0.0, 1, I, H)), quant(full(w_down, 1, H, I))
+    xs, rw = full(x, T, H), torch.full((T, 1), router_weight, device="cuda")
+    _, ctx = F.forward(cfg, ws, sched, xs, rw, *shared, wg[:2], wu[:2], wd[:2])
+    rows = ctx.gate_routed[0].shape[0]
+    ctx = dataclasses.replace(ctx, gate_routed=quant(full(gate, rows, I))[:2], up_routed=quant(full(up, rows, I))[:2])
+    grads = F.backward(cfg, ws, sched, ctx, full(grad_output, T, H), xs, rw, *shared, wg, wu, wd[2:])
+    torch.cuda.synchronize()
+    assert _C.check_status() == 0
+    return dict(zip(GRAD_KEYS, grads))
+
+
+def test_mxfp8_swiglu_backward_holds_gates_whose_exponential_is_near_the_largest_float():
+    # gate -88: silu is -5e-37 and the sigmoid 6e-39; an approximate reciprocal of 1 + exp(88) > 2^126 would be zero.
+    # E4M3 rounds a value by at most 2^-4.
+    T, H, gate = 512, 256, -88.0
+    d_hidden = 2.0 ** 100 * H
+    g = uniform_mxfp8_backward(T, H, x=1.0, gate=gate, up=1.0, w_down=2.0 ** 40, grad_output=2.0 ** 60, router_weight=1.0)
+    sig = 1.0 / (1.0 + np.exp(-gate))
+    for name, want in (("d_w_routed_up", gate * sig * d_hidden * T), ("d_w_routed_gate", sig * (1.0 + gate * (1.0 - sig)) * d_hidden * T)):
+        assert torch.all((g[name].double() - want).abs() <= abs(want) * 2.0 ** -4), (name, want, g[name].flatten()[:4])

@@ -169,6 +169,53 @@ def test_swiglu_fwd_bwd_vs_oracle(mods, limit):
     assert_close("row_grad", ref_rg[:512], rg[:512], (0.05 * float(ref_rg.abs().max()), 1e-3))
 
 
+@pytest.mark.parametrize("gate", [-87.0, -87.5, -88.0, -88.5])
+def test_swiglu_holds_gates_whose_exponential_is_near_the_largest_float(mods, gate):
+    """1 + exp(-gate) is between 2^125 and 2^128: silu (5e-37 in magnitude) and the sigmoid's derivative are far inside bf16's
+    range, and an approximate reciprocal would make them zero.  __expf is good to 2 + 1.17 * 88 units of 2^-24, the
+    rounding to bf16 to 2^-9: 2^-8 for both."""
+    _C, _ = mods
+    big = 2.0 ** 100
+    sig = 1.0 / (1.0 + np.exp(-gate))
+    full = lambda v: torch.full((256, 128), v, dtype=torch.bfloat16, device="cuda")
+    close = lambda got, want: torch.all((got.double() - want).abs() <= abs(want) * 2.0 ** -8)
+    assert close(_C.swiglu_fwd(full(gate), full(big)), gate * sig * big)
+    d_gate, d_up, _ = _C.swiglu_bwd(full(gate), full(1.0), full(big), None, None, False, None)
+    assert close(d_gate, sig * (1.0 + gate * (1.0 - sig)) * big) and close(d_up, gate * sig * big)
+    # the gate/up GEMM's epilogue: one column of x, so that gate and up are its weights
+    x = torch.zeros(256, 128, dtype=torch.bfloat16, device="cuda")
+    x[:, 0] = 1.0
+    Wg, Wu = (torch.zeros(1, 128, 128, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    Wg[:, :, 0], Wu[:, :, 0] = gate, big
+    g, u, h = (torch.empty(256, 128, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    _C.grouped_gemm(1, x, Wg, g, G=1, N=128, K=128, B2=Wu, D2=u, D3=h)
+    torch.cuda.synchronize()
+    assert torch.all(g == gate) and close(h, gate * sig * big)
+
+
+def test_gate_up_epilogue_rounds_like_the_ieee_quotient_for_every_gate_and_mantissa(mods):
+    """Every finite bf16 gate against every bf16 mantissa of up: the epilogue's hidden (approximate quotient, two units of fp32)
+    and the element-wise kernel's (IEEE quotient).  Before their last rounding the two are at most 2^-21 apart (2 x 2^-23 and
+    the product's rounding in both), so they may be neighbouring bf16 numbers where a tie lies between: 2^-21 of the 2^-8 between
+    two numbers is 2^-13 of the cases."""
+    _C, _ = mods
+    bits = torch.arange(65536, device="cuda", dtype=torch.int32)
+    gates = bits[(bits & 0x7F80) != 0x7F80].to(torch.int16).view(torch.bfloat16)
+    mantissas = (torch.arange(128, device="cuda", dtype=torch.int32) | 0x3F80).to(torch.int16).view(torch.bfloat16)
+    rows = gates.numel()                                   # 255 * 256
+    x = torch.zeros(rows, 128, dtype=torch.bfloat16, device="cuda")
+    x[:, 0], x[:, 1] = gates, 1.0
+    Wg, Wu = (torch.zeros(1, 128, 128, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    Wg[0, :, 0], Wu[0, :, 1] = 1.0, mantissas
+    g, u, h = (torch.empty(rows, 128, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    _C.grouped_gemm(1, x, Wg, g, G=1, N=128, K=128, B2=Wu, D2=u, D3=h)
+    want = _C.swiglu_fwd(g, u)
+    torch.cuda.synchronize()
+    assert torch.equal(g, gates[:, None].expand(rows, 128)) and torch.equal(u, mantissas[None].expand(rows, 128))
+    apart = (h.view(torch.int16).int() - want.view(torch.int16).int()).abs()      # (same sign: a distance in bf16 numbers)
+    assert int(apart.max()) <= 1 and int(apart.sum()) <= apart.numel() * 2.0 ** -13
+
+
 # ------------------------------------------------------------------ dispatch / combine (EP = 1 path of the peer kernels)
 def test_dispatch_and_combine_rows_single_rank(mods):
     _C, ops = mods
