@@ -93,7 +93,7 @@ __global__ void swiglu_bwd_kernel(const uint4* __restrict__ gate, const uint4* _
                 float dg0, du0, dg1, du1;
                 const float h0 = swiglu_bwd_one(gf.x, uf.x, df.x, c, &dg0, &du0);
                 const float h1 = swiglu_bwd_one(gf.y, uf.y, df.y, c, &dg1, &du1);
-                partial += df.x * h0 + df.y * h1;
+                partial += df.x * inv_w * h0 + df.y * inv_w * h1;      // (d_hidden * hidden alone can be below fp32's range)
                 ogp[k] = pack_bf16(dg0, dg1);
                 oup[k] = pack_bf16(du0, du1);
             }
@@ -103,7 +103,7 @@ __global__ void swiglu_bwd_kernel(const uint4* __restrict__ gate, const uint4* _
         if (row_grad_out) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) partial += __shfl_xor_sync(0xffffffffu, partial, o);
-            if (lane == 0) row_grad_out[row] = partial * inv_w;
+            if (lane == 0) row_grad_out[row] = partial;
         }
     }
 }

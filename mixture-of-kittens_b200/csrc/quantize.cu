@@ -211,8 +211,10 @@ __device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t v) {
 // grid (I/128, window rows/128), 256 threads: eight threads per row, 16 columns each, rows 32 apart in four trips; the next
 // trip's operands are in flight while this one's are worked on.  Every global access of a warp covers whole 128-byte
 // lines of four rows.  d_gate / d_up are quantised row-wise from registers and staged (two tiles) for the column-wise pass.
-// 135 k rows of 2048: 611 us (3.7 TB/s), bound by instructions at 24 warps per SM; 1188 us with a row per thread and 32 columns.
-__global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
+// The row gradient is summed in the order of the columns, so the lanes of a row hand the sum on, 32 registers of factors each:
+// two blocks per SM (three would spill: 1094 us).  135 k rows of 2048: 752 us (3.0 TB/s), bound by instructions, of which the
+// IEEE quotients take 110 us and the order of the sum 30; 1188 us with a row per thread and 32 columns.
+__global__ void __launch_bounds__(256, 2) swiglu_bwd_quant_kernel(
     const uint8_t* __restrict__ gate_q, const uint8_t* __restrict__ gate_sc, const uint8_t* __restrict__ up_q,
     const uint8_t* __restrict__ up_sc, const __nv_bfloat16* __restrict__ d_hidden, int64_t rows_cap, int64_t I,
     RowWindow win, Clamp c, const float* __restrict__ row_scale,
@@ -253,7 +255,7 @@ __global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
         const float inv_w = o.w > 0.0f ? 1.0f / o.w : 0.0f;
         const uint32_t gv[4] = {o.g.x, o.g.y, o.g.z, o.g.w}, uv[4] = {o.u.x, o.u.y, o.u.z, o.u.w};
         uint32_t wg[8], wu[8];
-        float partial = 0.0f;
+        float rg_a[16], rg_b[16];          // factors of the row gradient's terms
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const float2 gq = e4m3x2_to_float2(gv[i >> 1] >> ((i & 1) * 16));
@@ -276,7 +278,8 @@ __global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
                 const float dsilu = (1.0f - silu) * sig + silu;
                 dg[j] = g_ok ? dsilu * u * dhv[j] : 0.0f;
                 du[j] = u_ok ? silu * dhv[j] : 0.0f;
-                partial += dhv[j] * (silu * u);
+                rg_a[2 * i + j] = dhv[j] * inv_w;
+                rg_b[2 * i + j] = silu * u;
             }
             wg[i] = pack2(dg[0], dg[1]);
             wu[i] = pack2(du[0], du[1]);
@@ -285,10 +288,17 @@ __global__ void __launch_bounds__(256, 3) swiglu_bwd_quant_kernel(
         stage_16_columns(tdu, rr + 32 * k, seg, wu);
         quantize_16_columns(wg, dg_q + row * I + col, dg_sc + sc_off + 4 * k);
         quantize_16_columns(wu, du_q + row * I + col, du_sc + sc_off + 4 * k);
-        if (partials) {
+        if (partials) {      // the 64 columns of a half row in ascending order, handed from lane to lane; then the two halves
+            float run = 0.0f;
 #pragma unroll
-            for (int d = 4; d >= 1; d >>= 1) partial += __shfl_xor_sync(0xffffffffu, partial, d);
-            if (seg == 0) partials[row * (I >> 7) + blockIdx.x] = partial * inv_w;
+            for (int s = 0; s < 4; ++s) {      // (after step s the first s + 1 lanes of a half row hold their final sums)
+                const float left = __shfl_up_sync(0xffffffffu, run, 1);
+                run = (seg & 3) ? left : 0.0f;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) run = fmaf(rg_a[i], rg_b[i], run);
+            }
+            const float upper = __shfl_down_sync(0xffffffffu, run, 4);
+            if (seg == 3) partials[row * (I >> 7) + blockIdx.x] = run + upper;
         }
     }
     __syncthreads();

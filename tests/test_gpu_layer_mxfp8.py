@@ -160,3 +160,11 @@ def test_mxfp8_swiglu_backward_holds_gates_whose_exponential_is_near_the_largest
     sig = 1.0 / (1.0 + np.exp(-gate))
     for name, want in (("d_w_routed_up", gate * sig * d_hidden * T), ("d_w_routed_gate", sig * (1.0 + gate * (1.0 - sig)) * d_hidden * T)):
         assert torch.all((g[name].double() - want).abs() <= abs(want) * 2.0 ** -4), (name, want, g[name].flatten()[:4])
+
+
+def test_mxfp8_router_gradient_of_a_tiny_weight():
+    # d_hidden * hidden is 2^-62 * 2^-93, below fp32's range; with the router weight 2^-100 divided out of each term first the
+    # gradient is I * 2^-55.  Powers of two throughout; silu of 2^-46 is half of it.
+    g = uniform_mxfp8_backward(x=1.0, gate=2.0 ** -46, up=2.0 ** -46, w_down=2.0 ** -30, grad_output=2.0 ** 60, router_weight=2.0 ** -100)
+    want = 128 * 2.0 ** -55
+    assert torch.all((g["d_router_weights"].double() - want).abs() <= want * 2.0 ** -20), g["d_router_weights"][:4]

@@ -216,6 +216,18 @@ def test_gate_up_epilogue_rounds_like_the_ieee_quotient_for_every_gate_and_manti
     assert int(apart.max()) <= 1 and int(apart.sum()) <= apart.numel() * 2.0 ** -13
 
 
+def test_router_gradient_of_a_tiny_weight(mods):
+    """d_hidden carries the router weight, which is divided out again: the terms are formed after the division, so that
+    d_hidden * hidden below fp32's range (here 2^-123 * 2^-29) is not lost.  All powers of two but silu, 2^-15 (1 + 2^-15): bf16's
+    rounding plays no part, and the sum over 256 columns is good to 2^-13."""
+    _C, _ = mods
+    full = lambda v: torch.full((256, 256), v, dtype=torch.bfloat16, device="cuda")
+    w = torch.full((256,), 2.0 ** -123, device="cuda")
+    _, _, got = _C.swiglu_bwd(full(2.0 ** -14), full(2.0 ** -14), full(2.0 ** -123), None, w, True, None)
+    want = 256 * 2.0 ** -29
+    assert torch.all((got.double() - want).abs() <= want * 2.0 ** -13)
+
+
 # ------------------------------------------------------------------ dispatch / combine (EP = 1 path of the peer kernels)
 def test_dispatch_and_combine_rows_single_rank(mods):
     _C, ops = mods
