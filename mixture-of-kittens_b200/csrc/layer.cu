@@ -132,7 +132,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_bf16(const mokb_fwd_bf16_arg
         }
         // dispatch: pull every scheduled row from its home rank, in row order
         MOKB_TRY(dispatch_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
-                                    x_routed, nullptr, nullptr, comm_blocks, s_in, flags ? s.win_ready : nullptr, nullptr, nullptr, routes, a->status,
+                                    x_routed, nullptr, nullptr, m == 0 ? comm_blocks : lone_pull_block_count(), s_in, flags ? s.win_ready : nullptr, nullptr, nullptr, routes, a->status,
                                     flags ? s.ticket : nullptr, chunk));
         if (overlap) MOKB_CUDA(cudaEventRecord(as->join1, s_in));
 
@@ -226,7 +226,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_bf16(const mokb_bwd_bf16_arg
         // replay (later macrobatches only): pull x again; the saved context holds macrobatch 0
         if (m > 0)
             MOKB_TRY(dispatch_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
-                                        x_routed, nullptr, nullptr, comm_blocks, s_in, nullptr, nullptr, nullptr, routes, a->status));
+                                        x_routed, nullptr, nullptr, lone_pull_block_count(), s_in, nullptr, nullptr, nullptr, routes, a->status));
         if (overlap) MOKB_CUDA(cudaEventRecord(as->join1, s_in));     // the replayed x is in place
         // reverse combine: pull d_y rows, scaled by the route's router weight; in macrobatch 0 the first routed GEMM is one
         // launch that starts each window when the window's rows have arrived

@@ -49,6 +49,12 @@ inline int quant_comm_block_count(int num_comm_sms) {
     return wanted < sm_count() ? wanted : sm_count();
 }
 
+// A pull with nothing beside it -- rows of a later macrobatch, which the next GEMM waits for as a whole -- takes the whole chip:
+// four blocks per SM, as many as are resident of the quantising pull.  (Training with two or three populated macrobatches, MXFP8:
+// 16384 tokens, 32 experts of 7168 x 2048, 31.4 -> 30.3 ms; 8192 tokens, 4096 x 1536, 7.95 -> 7.60 ms; BF16 within noise.  Sixteen
+// blocks per SM cost the empty macrobatches 5 us each.)
+inline int lone_pull_block_count() { return 4 * sm_count(); }
+
 inline size_t scratch_bytes(int capacity, int E_l, int MB) {
     const size_t nm = macrobatches(capacity, MB);
     return align256((E_l + 1) * 4) + 512 + align256(nm * 4) + 2 * align256(nm * (E_l + 1) * 4) +

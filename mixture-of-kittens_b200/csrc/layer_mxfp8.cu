@@ -144,7 +144,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_fwd_mxfp8(const mokb_fwd_mxfp8_a
         // dispatch, in row order: the pull quantises every row along its columns (what the GEMM reads) and along tokens
         // (for the weight gradients of the backward pass) and counts the rows that have arrived, window by window
         MOKB_TRY(pull_quant_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
-                                      nullptr, nullptr, v.x_fp8, v.x_sc, v.x_fp8_t, v.x_sc_t, MB, comm_blocks, s_in,
+                                      nullptr, nullptr, v.x_fp8, v.x_sc, v.x_fp8_t, v.x_sc_t, MB, m == 0 ? comm_blocks : lone_pull_block_count(), s_in,
                                       flags ? s.ticket : nullptr, s.win_ready, chunk, routes, a->status));
         if (overlap) MOKB_CUDA(cudaEventRecord(as->join1, s_in));
 
@@ -255,7 +255,7 @@ extern "C" int mokb_dispatch_mlp_swiglu_combine_bwd_mxfp8(const mokb_bwd_mxfp8_a
         }
         if (m > 0)         // replay: pull x again and quantise it both ways
             MOKB_TRY(pull_quant_rows_impl(a->x_ptrs_host, a->ep_size, a->peer_rank, a->peer_token_idx, s.n_rows, C, lo, hi, a->topk, H,
-                                          nullptr, nullptr, v.x_fp8, v.x_sc, v.x_fp8_t, v.x_sc_t, MB, comm_blocks, s_in, nullptr, nullptr, 0,
+                                          nullptr, nullptr, v.x_fp8, v.x_sc, v.x_fp8_t, v.x_sc_t, MB, lone_pull_block_count(), s_in, nullptr, nullptr, 0,
                                           routes, a->status));
         if (overlap) MOKB_CUDA(cudaEventRecord(as->join1, s_in));     // the replayed x is in place
         // reverse combine: pull d_y rows scaled by the route's router weight and quantise them both ways (macrobatch 0: in
