@@ -468,7 +468,10 @@ int mokb_dispatch_rows_window(const uint64_t* src_ptrs_host, int ep_size, const 
                               int32_t* done_counter, void* q_out, void* q_sc_out, int64_t index_limit, int32_t* status,
                               void* stream);
 /* The pull that the MXFP8 layer uses: the rows in both MXFP8 forms (q [max_rows, hidden] + sc along columns, qt [hidden, t_rows]
- * + sct along rows; hidden a multiple of 256), the bf16 rows themselves are not stored.  With a ticket (device int32, zero)
+ * + sct along rows; hidden a multiple of 256), the bf16 rows themselves are not stored.  max_rows, row_begin, row_end and t_rows
+ * are multiples of 128, and the rows of the window fit t_rows (row r lies in token column r; a buffer that holds rows from
+ * another one on is passed moved back).  *num_rows is a multiple of 256 in every schedule of this library; where it is not, the
+ * rows up to the next multiple of 32 are written as padding (zeros) and none beyond.  With a ticket (device int32, zero)
  * the launch takes the rows in order and raises window_ready[w] by hidden / 32 per 256 rows of window w. */
 int mokb_dispatch_rows_quant(const uint64_t* src_ptrs_host, int ep_size, const int32_t* peer_rank, const int32_t* peer_token_idx,
                              const int32_t* num_rows, int max_rows, int row_begin, int row_end, int row_divisor, int64_t hidden,

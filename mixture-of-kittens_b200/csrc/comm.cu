@@ -611,6 +611,10 @@ int pull_quant_rows_impl(const uint64_t* src_ptrs_host, int ep_size, const int32
     MOKB_REQUIRE(ep_size >= 1 && ep_size <= MOKB_MAX_EP && peer_rank && peer_token_idx && q && sc && qt && sct, "pull_quant_rows: null pointer");
     MOKB_REQUIRE(hidden > 0 && hidden % kQuantCols == 0 && row_divisor >= 1 && row_begin >= 0 && row_begin <= row_end && row_begin % 128 == 0 && t_rows % 128 == 0,
                  "pull_quant_rows: bad sizes");
+    // a warp stores 32 rows and 32 token columns at a time, also where the device's row count ends inside of them
+    MOKB_REQUIRE(max_rows >= 0 && max_rows % 128 == 0 && row_end % 128 == 0, "pull_quant_rows: max_rows and row_end must be multiples of 128");
+    MOKB_REQUIRE((row_end < max_rows ? row_end : max_rows) - row_begin <= t_rows, "pull_quant_rows: %d rows do not fit the %lld token columns",
+                 (row_end < max_rows ? row_end : max_rows) - row_begin, static_cast<long long>(t_rows));
     MOKB_REQUIRE((reinterpret_cast<uintptr_t>(q) & 1) == 0 && (reinterpret_cast<uintptr_t>(qt) & 31) == 0, "pull_quant_rows: outputs not aligned");
     MOKB_REQUIRE(ticket == nullptr || (window_ready && window_rows > 0 && window_rows % 256 == 0), "pull_quant_rows: a ticket needs windows");
     MOKB_REQUIRE(index_limit >= 0 && index_limit <= INT32_MAX && (index_limit == 0 || status != nullptr), "pull_quant_rows: bad index limit");

@@ -37,3 +37,17 @@ def test_argument_errors_without_a_gpu():
     assert rc == -1 and b"null input" in _C._last_error()
     rc = lib.mokb_schedule(None, 1, 512, 2, 4, 2048, 0, None, None, None, None, None, None, None)
     assert rc == -1 and b"null pointer" in _C._last_error()
+
+
+def test_the_quantising_pull_refuses_rows_that_its_stores_would_leave():
+    """Its warps store 32 rows and 32 token columns at a time: checked before anything is launched (the addresses are never read)."""
+    from mok import _C
+    src = (ctypes.c_uint64 * 1)(4096)
+    def call(max_rows, row_begin, row_end, t_rows):
+        vp = lambda: ctypes.c_void_p(4096)
+        return _C.lib.mokb_dispatch_rows_quant(src, 1, vp(), vp(), None, max_rows, row_begin, row_end, 1, 256, None, None, vp(), vp(), vp(), vp(),
+                                               t_rows, 0, None, None, 0, 0, None, None)
+    for args, why in (((100, 0, 128, 128), b"multiples of 128"), ((256, 0, 100, 256), b"multiples of 128"), ((-128, 0, 128, 128), b"multiples of 128"),
+                      ((256, 0, 256, 128), b"do not fit"), ((512, 128, 512, 256), b"do not fit")):
+        assert call(*args) == -1 and why in _C._last_error(), args
+    assert call(0, 0, 0, 128) == 0 and call(256, 256, 512, 256) == 0      # no rows: nothing to do

@@ -230,6 +230,28 @@ def test_the_quantising_pull_matches_the_pull_and_the_quantiser(R, T, K, H, scal
     assert int((torch.from_numpy(pr[:N]) < 0).sum()) > 0          # the case has padding rows
 
 
+@pytest.mark.parametrize("N", [100, 128, 257])
+def test_the_quantising_pull_with_a_row_count_inside_a_group_of_32(N):
+    """Rows past the device's count: those of the last group of 32 are padding (zeros), the others stay untouched."""
+    from mok import _C, ops
+    C, H = 384, 256
+    x = torch.randn(C, H, generator=torch.Generator().manual_seed(98)).to(torch.bfloat16).cuda()
+    prd, ptd = torch.zeros(C, dtype=torch.int32, device="cuda"), torch.arange(C, dtype=torch.int32, device="cuda")
+    full = lambda *shape: torch.full(shape, 77, dtype=torch.uint8, device="cuda")
+    q, sc, qt, sct = full(C, H), full(C // 128, H // 128, 32, 16), full(H, C), full(H // 128, C // 128, 32, 16)
+    _C.dispatch_rows_quant([x.data_ptr()], prd, ptd, torch.tensor([N], dtype=torch.int32, device="cuda"), C, 1, H, q, sc, qt, sct, blocks=2)
+    torch.cuda.synchronize()
+    assert _C.check_status() == 0
+    live = (N + 31) // 32 * 32
+    rows = x.clone()
+    rows[N:] = 0
+    want = ops.mxfp8_quantize(rows, True, True)
+    assert torch.equal(q[:live], want[0].view(torch.uint8)[:live]) and torch.equal(qt[:, :live], want[2].view(torch.uint8)[:, :live])
+    assert torch.equal(O.unpack_scales(sc.cpu())[:live], O.unpack_scales(want[1].cpu())[:live])
+    assert torch.equal(O.unpack_scales(sct.cpu())[:, :live // 32], O.unpack_scales(want[3].cpu())[:, :live // 32])
+    assert (q[live:] == 77).all() and (qt[:, live:] == 77).all()
+
+
 def test_transposed_only_quantiser_matches_the_two_way_quantiser():
     from mok import ops
     g = torch.Generator().manual_seed(92)
