@@ -25,7 +25,7 @@
  *     on schedule overflow, csrc/scheduler.cuh:86, and spins without bound,
  *     csrc/utils.cuh:274-277); after MOKB_ST_FLAG_TIMEOUT words 1..3 say which wait
  *     ran out (1 = a GEMM on a dispatch window, 2 = a down tile on its gate/up tiles,
- *     3 = combine on a GEMM window; the counter's index; value seen << 16 | target).
+ *     3 = combine on a GEMM window; the counter's index; value seen << 16 | target, at most 32767 and 65535).
  *     The words are only ever written when something went wrong; the caller zeroes them.
  */
 #ifndef MOK_B200_H

@@ -202,7 +202,8 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
 // the TMA reads this thread issues next
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
-// `kind` / `index` say which counter it was (status words 1..3, for diagnosis: kind, index, value seen << 16 | target)
+// `kind` / `index` say which counter it was (status words 1..3, for diagnosis: kind, index, value seen << 16 | target, both
+// held at their largest: a window of many rows counts more arrivals than 16 bits hold)
 enum { kWaitWindowReady = 1, kWaitBlockDone = 2, kWaitWindowDone = 3 };
 
 __device__ __forceinline__ bool flag_wait(const int* flag, int target, volatile int* abort_flag, int* status, int kind, int index) {
@@ -220,7 +221,7 @@ __device__ __forceinline__ bool flag_wait(const int* flag, int target, volatile 
                 if (status && atomicCAS(status, 0, MOKB_ST_FLAG_TIMEOUT) == 0) {
                     status[1] = kind;
                     status[2] = index;
-                    status[3] = (seen << 16) | (target & 0xFFFF);
+                    status[3] = (min(max(seen, 0), 0x7FFF) << 16) | min(target, 0xFFFF);
                 }
                 return false;
             }

@@ -238,7 +238,8 @@ _LAST_DETAIL = [0, 0, 0, 0]
 
 
 def status_detail() -> list[int]:
-    """The four status words as the last check_status() read them: [code, kind, index, value seen << 16 | target]."""
+    """The four status words as the last check_status() read them: [code, kind, index, value seen << 16 | target] (at most
+    32767 and 65535)."""
     return list(_LAST_DETAIL)
 
 

@@ -173,6 +173,20 @@ def test_a_gemm_whose_window_never_becomes_ready_gives_up_with_a_status_code():
     assert all(torch.equal(a, b) for a, b in zip(ref, (gate, up, hid, y)))
 
 
+def test_the_diagnosis_of_a_wait_holds_counts_of_more_than_16_bits():
+    # 40000 of 70000 arrivals seen: both halves of the word stay at their largest value instead of wrapping
+    from mok import _C
+    p = problem([512], 256, 128, seed=75)
+    gate, up, hid, _ = outputs(p, fill=5.0)
+    ready = torch.full((1,), 40000, dtype=torch.int32, device="cuda")
+    _C.grouped_gemm(1, p["x"], p["Wg"], gate, group_of_block=p["gob"], G=1, N=128, K=256, B2=p["Wu"], D2=up, D3=hid, window_rows=512,
+                    win_ready=ready, win_ready_target=70000)
+    torch.cuda.synchronize()
+    assert _C.check_status() == _C.ST_FLAG_TIMEOUT
+    assert _C.status_detail() == [_C.ST_FLAG_TIMEOUT, 1, 0, 32767 << 16 | 65535]
+    assert torch.all(gate == 5.0)
+
+
 def test_a_combine_whose_rows_never_arrive_gives_up_and_copies_nothing():
     from mok import _C
     rows, H = 512, 256
