@@ -88,16 +88,11 @@ int combine_rows_impl(const void* src, const uint64_t* dst_ptrs_host, int ep_siz
                       const int32_t* wait_counter = nullptr, int arrivals_per_row_block = 0, int32_t* status = nullptr,
                       int64_t index_limit = 0);
 
-// MXFP8 codec launchers (quantize.cu).  Rows [row_begin, min(row_end, *num_rows)) are processed (row_end = 0: all
-// M / rows_cap rows; `num_rows` is a device pointer, optional).  Row numbers are the caller's: a buffer holding only
-// rows [first, first + M) is passed with every pointer moved back by `first` rows (transposed tensors: by `first`
-// bytes, scale tensors: by first / 128 tiles along the row axis), and M / rows_cap stays the buffer's own row count,
+// SwiGLU backward of the MXFP8 layer (quantize.cu).  Rows [row_begin, min(row_end, *num_rows)) are processed (row_end = 0: all
+// rows_cap rows; `num_rows` is a device pointer, optional).  Row numbers are the caller's: a buffer holding only
+// rows [first, first + rows_cap) is passed with every pointer moved back by `first` rows (transposed tensors: by `first`
+// bytes, scale tensors: by first / 128 tiles along the row axis), and rows_cap stays the buffer's own row count,
 // which is also the row stride of the transposed outputs.
-// On `blocks` CTAs (0 = as many as there are tiles, up to 16 per SM); `done_counter`: every block of the launch adds 1
-// (release) when it is through, so the window is quantised when the counter has grown by `blocks`.
-int quantize_impl(const void* x_bf16, int64_t E, int64_t M, int64_t N, const int32_t* num_rows, int row_begin, int row_end,
-                  void* x_fp8, void* x_sc, void* x_fp8_t, void* x_sc_t, cudaStream_t stream, int blocks = 0,
-                  int32_t* done_counter = nullptr);
 int swiglu_bwd_quant_impl(const void* gate_q, const void* gate_sc, const void* up_q, const void* up_sc, const void* d_hidden,
                           int64_t rows_cap, int64_t I, const int32_t* num_rows, int row_begin, int row_end, int has_limit, float limit,
                           const float* row_scale, void* dg_q, void* dg_sc, void* dg_qt, void* dg_sct,

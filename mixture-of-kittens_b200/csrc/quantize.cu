@@ -95,16 +95,14 @@ __device__ __forceinline__ bool tile_in_window(const RowWindow& w, int64_t* r0) 
     return *r0 < live;
 }
 
-// 256 threads per block; the blocks of the launch walk the 128 x 128 tiles of the window (column tiles fastest).
-// 32 x 2048 x 7168 both ways: 455 us (4.2 TB/s; 508 us with 32 columns of a row per thread), as much for one form alone (4.3 TB/s);
-// a fourth block per SM (64 registers) changes nothing.
+// 256 threads per block; the blocks of the launch walk the 128 x 128 tiles (column tiles fastest).
+// 32 x 2048 x 7168 both ways: 341 us (5.6 TB/s), row-wise alone 229 (6.2).  The SM's default split between L1 and shared memory is
+// part of that: with the GEMMs' split (all shared memory, as the pulls that run beside them have it) 458 and 322 us.
 __global__ void __launch_bounds__(256) quantize_kernel(const __nv_bfloat16* __restrict__ x, int64_t E, int64_t M, int64_t N,
-                                                       RowWindow win,
                                                        uint8_t* __restrict__ q, uint8_t* __restrict__ sc,
-                                                       uint8_t* __restrict__ qt, uint8_t* __restrict__ sct, int32_t* done_counter) {
+                                                       uint8_t* __restrict__ qt, uint8_t* __restrict__ sct) {
     __shared__ __align__(16) uint32_t tile[TILE_WORDS];
-    const int live = win.num_rows ? min(max(*win.num_rows, 0), win.end) : win.end;
-    const int64_t row_tiles = live > win.begin ? (live - win.begin + TILE - 1) / TILE : 0;
+    const int64_t row_tiles = M / TILE;
     const int64_t col_tiles = N / TILE;
     const int64_t ntiles = E * row_tiles * col_tiles;
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -112,7 +110,7 @@ __global__ void __launch_bounds__(256) quantize_kernel(const __nv_bfloat16* __re
         const int64_t rem = t - e * row_tiles * col_tiles;
         const int64_t rt = rem / col_tiles;
         const int64_t c0 = (rem - rt * col_tiles) * TILE;
-        const int64_t r0 = win.begin + rt * TILE;
+        const int64_t r0 = rt * TILE;
         const int seg = threadIdx.x & 7, rr = threadIdx.x >> 3;      // 16 columns of rows rr, rr + 32, ..
         const __nv_bfloat16* src = x + (e * M + r0 + rr) * N + c0 + seg * 16;
         uint32_t val[4][8];
@@ -128,33 +126,21 @@ __global__ void __launch_bounds__(256) quantize_kernel(const __nv_bfloat16* __re
         if (qt) quantize_tile_cols(tile, qt, sct, e * N, r0, c0, M);
         __syncthreads();          // the tile is free for the next load
     }
-    if (done_counter) {      // one arrival per block of the launch (also those without tiles): the window is quantised
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            red_release_gpu_add(done_counter, 1);
-        }
-    }
 }
 
-// Column-wise ("transposed") quantisation only, for tensors whose row-wise form already exists (the dispatch kernel
-// writes it as the rows arrive): qt [N, M] + scales from x [M, N].  No shared memory and at most 64 registers, so that
-// two blocks of 128 threads fit on an SM beside any of the GEMM kernels (the MXFP8 GEMM leaves less than 8 KB of
-// shared memory and 4096 registers per SM quarter) and the pass runs under the GEMM instead of after it.  A lane owns
-// a pair of adjacent columns over a block of 32 rows: its 32 loads are independent, and a warp's load of one row is
-// one 128-byte line.  Same arithmetic as quantize_tile_cols.
+// Column-wise ("transposed") quantisation of one matrix only, for callers that ask for nothing else: qt [N, M] + scales from
+// x [M, N].  No shared memory and at most 64 registers.  A lane owns a pair of adjacent columns over a block of 32 rows: its 32
+// loads are independent, and a warp's load of one row is one 128-byte line.  Same arithmetic as quantize_tile_cols.
 constexpr int CTILE_COLS = 64;
-__global__ void __maxnreg__(64) quantize_cols_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int64_t N, RowWindow win,
+__global__ void __maxnreg__(64) quantize_cols_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int64_t N,
                                                      uint8_t* __restrict__ qt, uint8_t* __restrict__ sct) {
-    const int live = win.num_rows ? min(max(*win.num_rows, 0), win.end) : win.end;
-    const int64_t row_tiles = live > win.begin ? (live - win.begin + TILE - 1) / TILE : 0;
     const int64_t col_tiles = N / CTILE_COLS;
-    const int64_t ntiles = row_tiles * col_tiles;
+    const int64_t ntiles = M / TILE * col_tiles;
     const int cp = threadIdx.x & 31, kb = threadIdx.x >> 5;      // a pair of adjacent columns, a block of 32 rows
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int64_t rt = t / col_tiles;
         const int64_t c0 = (t - rt * col_tiles) * CTILE_COLS;
-        const int64_t r0 = win.begin + rt * TILE + kb * 32;
+        const int64_t r0 = rt * TILE + kb * 32;
         const int64_t col = c0 + 2 * cp;
         const uint32_t* src = reinterpret_cast<const uint32_t*>(x + r0 * N + col);
         const int64_t pitch = N / 2;                             // 32-bit words per row
@@ -329,40 +315,6 @@ int check_window(const char* who, int row_begin, int* row_end, int64_t rows) {
 }
 }  // namespace
 
-int quantize_impl(const void* x_bf16, int64_t E, int64_t M, int64_t N, const int32_t* num_rows, int row_begin, int row_end,
-                  void* x_fp8, void* x_sc, void* x_fp8_t, void* x_sc_t, cudaStream_t stream, int blocks, int32_t* done_counter) {
-    TraceScope trace(stream, "quantize", row_begin);
-    MOKB_REQUIRE(x_bf16 != nullptr, "mxfp8_quantize: null input");
-    MOKB_REQUIRE(E > 0 && M > 0 && N > 0 && M % 128 == 0 && N % 128 == 0, "mxfp8_quantize: M and N must be positive multiples of 128");
-    MOKB_REQUIRE((x_fp8 == nullptr) == (x_sc == nullptr) && (x_fp8_t == nullptr) == (x_sc_t == nullptr),
-                 "mxfp8_quantize: data and scale outputs go together");
-    MOKB_REQUIRE(x_fp8 || x_fp8_t, "mxfp8_quantize: at least one quantised layout must be requested");
-    MOKB_REQUIRE(aligned32(x_bf16) && aligned32(x_fp8) && aligned32(x_fp8_t), "mxfp8_quantize: tensors must be 32-byte aligned");
-    MOKB_TRY(check_window("mxfp8_quantize", row_begin, &row_end, M));
-    if (row_begin == row_end) return MOKB_OK;
-    if (x_fp8 == nullptr && E == 1 && done_counter == nullptr) {
-        const int64_t ct = ((row_end - row_begin) / 128) * (N / CTILE_COLS);
-        if (blocks <= 0) blocks = static_cast<int>(ct < 8ll * sm_count() ? ct : 8ll * sm_count());
-        share_sms_with_gemm<quantize_cols_kernel>();
-        quantize_cols_kernel<<<static_cast<unsigned>(blocks), 128, 0, stream>>>(static_cast<const __nv_bfloat16*>(x_bf16), M, N,
-                                                                                RowWindow{num_rows, row_begin, row_end},
-                                                                                static_cast<uint8_t*>(x_fp8_t), static_cast<uint8_t*>(x_sc_t));
-        MOKB_CUDA(cudaGetLastError());
-        note_launch();
-        return MOKB_OK;
-    }
-    const int64_t tiles = E * ((row_end - row_begin) / 128) * (N / 128);
-    if (blocks <= 0) blocks = static_cast<int>(tiles < 16ll * sm_count() ? tiles : 16ll * sm_count());
-    share_sms_with_gemm<quantize_kernel>();
-    quantize_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x_bf16), E, M, N,
-                                                                       RowWindow{num_rows, row_begin, row_end},
-                                                                       static_cast<uint8_t*>(x_fp8), static_cast<uint8_t*>(x_sc),
-                                                                       static_cast<uint8_t*>(x_fp8_t), static_cast<uint8_t*>(x_sc_t), done_counter);
-    MOKB_CUDA(cudaGetLastError());
-    note_launch();
-    return MOKB_OK;
-}
-
 int swiglu_bwd_quant_impl(const void* gate_q, const void* gate_sc, const void* up_q, const void* up_sc, const void* d_hidden,
                           int64_t rows_cap, int64_t I, const int32_t* num_rows, int row_begin, int row_end, int has_limit, float limit,
                           const float* row_scale, void* dg_q, void* dg_sc, void* dg_qt, void* dg_sct,
@@ -403,6 +355,27 @@ int swiglu_bwd_quant_impl(const void* gate_q, const void* gate_sc, const void* u
 using namespace mokb;
 
 extern "C" int mokb_mxfp8_quantize(const void* x_bf16, int64_t E, int64_t M, int64_t N,
-                                   void* x_fp8, void* x_sc, void* x_fp8_t, void* x_sc_t, void* stream) {
-    return quantize_impl(x_bf16, E, M, N, nullptr, 0, 0, x_fp8, x_sc, x_fp8_t, x_sc_t, static_cast<cudaStream_t>(stream));
+                                   void* x_fp8, void* x_sc, void* x_fp8_t, void* x_sc_t, void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    TraceScope trace(stream, "quantize");
+    MOKB_REQUIRE(x_bf16 != nullptr, "mxfp8_quantize: null input");
+    MOKB_REQUIRE(E > 0 && M > 0 && N > 0 && M % 128 == 0 && N % 128 == 0, "mxfp8_quantize: M and N must be positive multiples of 128");
+    MOKB_REQUIRE((x_fp8 == nullptr) == (x_sc == nullptr) && (x_fp8_t == nullptr) == (x_sc_t == nullptr),
+                 "mxfp8_quantize: data and scale outputs go together");
+    MOKB_REQUIRE(x_fp8 || x_fp8_t, "mxfp8_quantize: at least one quantised layout must be requested");
+    MOKB_REQUIRE(aligned32(x_bf16) && aligned32(x_fp8) && aligned32(x_fp8_t), "mxfp8_quantize: tensors must be 32-byte aligned");
+    if (x_fp8 == nullptr && E == 1) {
+        const int64_t ct = (M / 128) * (N / CTILE_COLS);
+        const unsigned blocks = static_cast<unsigned>(ct < 8ll * sm_count() ? ct : 8ll * sm_count());
+        quantize_cols_kernel<<<blocks, 128, 0, stream>>>(static_cast<const __nv_bfloat16*>(x_bf16), M, N, static_cast<uint8_t*>(x_fp8_t),
+                                                         static_cast<uint8_t*>(x_sc_t));
+    } else {
+        const int64_t tiles = E * (M / 128) * (N / 128);
+        const unsigned blocks = static_cast<unsigned>(tiles < 16ll * sm_count() ? tiles : 16ll * sm_count());
+        quantize_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x_bf16), E, M, N, static_cast<uint8_t*>(x_fp8),
+                                                    static_cast<uint8_t*>(x_sc), static_cast<uint8_t*>(x_fp8_t), static_cast<uint8_t*>(x_sc_t));
+    }
+    MOKB_CUDA(cudaGetLastError());
+    note_launch();
+    return MOKB_OK;
 }
