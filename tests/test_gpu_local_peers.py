@@ -194,8 +194,13 @@ def test_dispatch_quantises_the_rows_it_pulls_like_the_quantiser(R, T, K, H, sca
     assert int((torch.from_numpy(pr[:N]) < 0).sum()) > 0          # the case has padding rows
 
 
-@pytest.mark.parametrize("R,T,K,H,scaled,window", [(2, 512, 2, 256, False, 256), (4, 512, 4, 512, True, 0), (2, 512, 2, 7168, True, 512)])
-def test_the_quantising_pull_matches_the_pull_and_the_quantiser(R, T, K, H, scaled, window):
+@pytest.mark.parametrize("R,T,K,H,scaled,window,blocks", [
+    (2, 512, 2, 256, False, 256, 16), (4, 512, 4, 512, True, 0, 16), (2, 512, 2, 7168, True, 512, 16),
+    (2, 1024, 2, 1280, True, 512, 2), (2, 1024, 2, 1280, False, 0, 2),           # units of 1024 columns, the last one of 256
+    (2, 1024, 2, 2816, False, 1024, 2),                                          # and of 768
+    (2, 1024, 2, 1792, True, 256, 6),                                            # units of 512 columns, the last one of 256
+])
+def test_the_quantising_pull_matches_the_pull_and_the_quantiser(R, T, K, H, scaled, window, blocks):
     """Both MXFP8 forms straight from the pulled registers against the bf16 pull followed by the two-way quantiser: bytes and
     scales identical, padding rows included; by ticket also the count of arrivals per window."""
     from mok import _C, ops
@@ -218,7 +223,7 @@ def test_the_quantising_pull_matches_the_pull_and_the_quantiser(R, T, K, H, scal
     qt, sct = torch.zeros(H, C, **u8), torch.zeros(H // 128, C // 128, 32, 16, **u8)
     ready = torch.zeros(C // (window or C) + 1, dtype=torch.int32, device="cuda")
     extra = dict(ticket=torch.zeros(1, dtype=torch.int32, device="cuda"), window_ready=ready, window_rows=window) if window else {}
-    _C.dispatch_rows_quant(xs, prd, ptd, ntd, C, K, H, q, sc, qt, sct, row_scale_ptrs=ws, row_scale_out=got_w, blocks=16, index_limit=T * K, **extra)
+    _C.dispatch_rows_quant(xs, prd, ptd, ntd, C, K, H, q, sc, qt, sct, row_scale_ptrs=ws, row_scale_out=got_w, blocks=blocks, index_limit=T * K, **extra)
     torch.cuda.synchronize()
     assert _C.check_status() == 0
     assert torch.equal(q[:N], want[0].view(torch.uint8)) and torch.equal(sc[:N // 128], want[1])

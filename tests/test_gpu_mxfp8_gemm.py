@@ -123,6 +123,30 @@ def test_mxfp8_gemm_gate_up_swiglu_quant_equals_the_unfused_sequence(limit):
         assert (got_s != ref_s).float().mean().item() < 0.01, name
 
 
+@pytest.mark.parametrize("offset", [1, 16])
+def test_mxfp8_gemm_gate_up_stores_the_token_wise_hidden_at_any_address(offset):
+    """hidden along tokens leaves 32 bytes at a time where its buffer is aligned to that, otherwise byte by byte: the same bytes,
+    and none outside."""
+    from mok import _C
+    rows, N, K = 512, 256, 128
+    g = torch.Generator().manual_seed(36)
+    Aq, As, _ = quant(torch.randn(rows, K, generator=g).to(torch.bfloat16))
+    Gq, Gs, _ = quant((torch.randn(1, N, K, generator=g) * 0.2).to(torch.bfloat16))
+    Uq, Us, _ = quant((torch.randn(1, N, K, generator=g) * 0.2).to(torch.bfloat16))
+    full = lambda *shape: torch.full(shape, 77, dtype=torch.uint8, device="cuda")
+    got = []
+    for off in (0, offset):
+        buffer = full(N * rows + 64)
+        scales = [full(rows // 128, N // 128, 32, 16) for _ in range(3)]
+        outs = [x for sc in scales for x in (full(rows, N), sc)] + [buffer[off:off + N * rows].view(N, rows), full(N // 128, rows // 128, 32, 16)]
+        _C.grouped_gemm_mxfp8(3, Aq, As, Gq, Gs, None, G=1, N=N, K=K, B2=Uq, B2_sc=Us, quantised_outputs=outs, t_rows=rows)
+        torch.cuda.synchronize()
+        assert _C.check_status() == 0
+        assert (buffer[:off] == 77).all() and (buffer[off + N * rows:] == 77).all()
+        got.append(outs)
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("cols_per_group,M,N", [([256], 128, 256), ([512, 0, 256], 256, 384), ([256, 1024], 384, 512)])
 def test_mxfp8_gemm_wgrad(cols_per_group, M, N):
     from mok import _C
@@ -201,7 +225,9 @@ def test_mxfp8_gemm_wgrad_leaves_out_the_padding_tokens_it_is_told_about():
 
 
 @pytest.mark.parametrize("rows_per_group,H,I,window,push", [([512, 256, 0, 768], 512, 384, 512, False),
-                                                            ([2048, 512, 3072], 768, 512, 1024, True)])
+                                                            ([2048, 512, 3072], 768, 512, 1024, True),
+                                                            # the down tiles follow six super-groups behind, the last one partial
+                                                            ([256] * 35 + [1536], 1024, 384, 512, False)])
 def test_mxfp8_fused_forward_equals_the_two_launches_bit_for_bit(rows_per_group, H, I, window, push):
     """Mode 4 (gate|up + SwiGLU + quantisation tiles and the down tiles of the same rows in one persistent launch, tied
     by counters) against mode 3 followed by mode 0; with `push`, the down rows go to a (local) peer buffer instead."""
