@@ -11,10 +11,12 @@
  *   - all pointers are device pointers on the current CUDA device unless the
  *     name ends in `_host`; tensors are contiguous, row-major;
  *   - `stream` is a cudaStream_t passed as void*; work is enqueued, never
- *     synchronised: no entry point blocks the host.  The layer entry points also use two
- *     streams of their own per device (the pulls, at high priority, and the token-wise MXFP8
- *     copies, at low priority), forked from and joined back into `stream` with events inside the
- *     call, so that to the caller everything is ordered on `stream`;
+ *     synchronised: no entry point blocks the host.  The layer entry points also use one
+ *     stream of their own per device (the pulls, at high priority), forked from and joined back
+ *     into `stream` with events inside the call, so that to the caller everything is ordered on
+ *     `stream`;
+ *   - schedules are those of mokb_schedule: every expert's segment, and so the row count, is a
+ *     multiple of 256 rows;
  *   - "peer pointer lists" (`*_ptrs_host`) are host arrays of `ep_size` device
  *     addresses, index = EP rank, as produced by a symmetric-memory rendezvous
  *     (mok/functional.py:224 of the reference);

@@ -305,9 +305,10 @@ __device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap* t, uin
     else tma_load_2d(dst, t, bar, c0, c1);
 }
 
-// 128 registers per thread at most: registers are handed out per SM quarter (16 K each), a CTA's six warps put two
-// on a quarter, and the dispatch / quantise blocks that run beside the GEMM (eight warps of 56 registers, two per
-// quarter) must still fit there -- a GEMM that waits for their rows on an SM they cannot enter would wait for ever.
+// 128 registers per thread at most: registers are handed out per SM quarter (16 K each), a CTA's six warps put at most two
+// on a quarter (a weight gradient's ten at most three, 12 K), and the pulls that run beside the GEMM must still fit there
+// (four warps a block, one per quarter: two blocks at 64 registers a thread, one of the quantising pull at 128) -- a GEMM that
+// waits for their rows on an SM they cannot enter would wait for ever.
 template <int MODE, int NCTA>
 __global__ void __maxnreg__(128)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,

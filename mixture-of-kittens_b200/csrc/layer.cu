@@ -9,7 +9,7 @@
 //                          { wait win_ready[w]; gate/up + SwiGLU tiles; down tiles, each after the gate/up tiles of its
 //                            256 rows (blk_done); the down epilogue stores every row into its home rank's combine buffer }
 //   backward  side stream: scaled dispatch of d_y, likewise
-//             caller     : prologue | shared backward (6 launches) | d_hidden = d_y * W_down (one launch, window by window)
+//             caller     : prologue | shared backward (4 launches) | d_hidden = d_y * W_down (one launch, window by window)
 //                          | SwiGLU backward | d_x = d_gate * W_gate + d_up * W_up, whose epilogue stores every row and its
 //                            router-weight gradient into the home rank's buffers | three weight gradients in one launch
 //
@@ -42,7 +42,8 @@ int get_async(Async** out) {
     MOKB_REQUIRE(dev >= 0 && dev < 64, "layer: device index %d out of range", dev);
     Async& a = g_async[dev];
     if (!a.ready) {
-        // s1 carries the pulls a waiting GEMM depends on: where both have blocks ready for the same free slot of an SM, the pull goes first
+        // s1 carries the pulls a waiting GEMM depends on: where its blocks and the GEMM's are ready for the same free slot of an SM, the
+        // pull goes first
         int prio_low = 0, prio_high = 0;
         MOKB_CUDA(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
         MOKB_CUDA(cudaStreamCreateWithPriority(&a.s1, cudaStreamNonBlocking, prio_high));

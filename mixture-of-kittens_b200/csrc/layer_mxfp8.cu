@@ -22,11 +22,9 @@ using namespace mokb;
 // SwiGLU + quantise) into the same buffers, accumulating the weight gradients.  Kernels address rows by
 // their schedule row number; a buffer's pointers are moved back by the macrobatch's first row.
 //
-// Overlap: macrobatch 0 of the forward is cut into row windows (minibatch_size rows): dispatch + quantise of
-// window c+1 and the combine of window c-1 run on the side streams while the GEMMs of window c run on the
-// caller's stream.  In the backward the d_y pull + quantisation comes in four windows behind the shared
-// expert's BF16 GEMMs, the first routed GEMM follows it window by window, and the d_x push overlaps the
-// weight gradients.
+// Overlap: the pull of macrobatch 0 runs on a side stream, in row order, and counts the rows that have arrived per window
+// of minibatch_size rows; beside it run the shared expert's BF16 GEMMs and then the first routed launch, which starts a
+// window when its rows are there.  Nothing is pushed beside the GEMMs: the epilogues store the rows at home.
 namespace mokb {
 namespace {
 

@@ -27,6 +27,9 @@ MAX_EP = ops.MAX_EP
 
 @dataclass(frozen=True, slots=True)
 class MoKConfig:
+    """The reference's six knobs.  `*_num_comm_sms` set how many threads pull rows (2048 per SM named), but never more than fit
+    beside the GEMMs that run at the same time: on 148 SMs every value from 20 on is the same launch in BF16, from 10 on in
+    MXFP8, the defaults among them."""
     fwd_num_comm_sms: int = 40
     bwd_num_comm_sms: int = 28
     minibatch_size: int = 4096
