@@ -112,8 +112,8 @@ int mokb_schedule(const int32_t* topk_all, int ep_size, int num_local_tokens, in
  *     call fails with MOKB_ERR_INVALID and a message that names the limit.
  *   - The first call on a device looks up the array's device address (once per device, with
  *     that device current); make that first call before any stream capture begins.
- *   - All calls on a device share the one array and find in it what the last call left; the
- *     entry point clears the part that must start at zero.  Two calls whose kernels overlap
+ *   - All calls on a device share the one array and find in it what the last call left; every
+ *     word that a call reads it has written before.  Two calls whose kernels overlap
  *     on the GPU (different streams, or different host threads) race on it: serialise them. */
 #define MOKB_SCHEDULE_NOALLOC_MAX_EXPERTS 1024
 int mokb_schedule_noalloc(const int32_t* topk_all, int ep_size, int num_local_tokens, int topk,

@@ -117,7 +117,8 @@ __device__ __forceinline__ void count_arrivals(int32_t* counter, int n) {
     }
 }
 
-// One warp per schedule row, 16- or 32-byte accesses, four loads in flight per lane.  QUANT (32-byte accesses only):
+// One warp per schedule row, 16- or 32-byte accesses, four loads in flight per lane.  QUANT (32-byte accesses only; for callers of
+// mokb_dispatch_rows_window that want the bf16 rows as well -- the MXFP8 layer pulls with pull_quant_kernel):
 // the row is also quantised along its columns from the registers it passes through -- a lane holds 16 consecutive
 // values, two neighbouring lanes one 32-value block (the reference quantises the tile it has just pulled,
 // csrc/megakernel/dispatch_combine.cuh:88-114; the values are those of quantize_kernel, byte for byte).
